@@ -453,7 +453,7 @@ cudaError_t encode_map(const float *d_map, int64_t n, cudaStream_t s, MapCodes *
         CK(cudaMalloc(&out->vals, sizeof(float) * (nd > 0 ? nd : 1)));
         values_k<<<blocks_for(nw), kB, 0, s>>>(bitmap, prefix, nw, out->vals);
         CK(cudaGetLastError());
-        CK(cudaMalloc(&out->codes8, sizeof(uint8_t) * (n > 0 ? n : 1)));
+        CK(cudaMalloc(&out->codes8, (size_t)(n > 0 ? n + 3 : 4) & ~size_t(3)));  // read as 32-bit words
         out->code_bits = bits;
         if (nd <= 65536) {
             CK(cudaMalloc(&out->codes, sizeof(uint16_t) * (n > 0 ? n : 1)));

@@ -140,6 +140,12 @@ void apply_options(grc_ctx *ctx) {
     g.Ruf[1] = (float)(g.R[7] / g.pxy);
     g.Rvf[0] = (float)(g.R[5] / g.pxz);
     g.Rvf[1] = (float)(g.R[8] / g.pxz);
+    g.rpxy = 1.0 / g.pxy;
+    g.rpxz = 1.0 / g.pxz;
+    g.Raf[0] = (float)(g.R[1] / (g.R[0] * g.pxy));
+    g.Raf[1] = (float)(g.R[2] / (g.R[0] * g.pxz));
+    g.beam_stop = g.bsy0 <= g.bsy1 && g.bsy1 >= 1.0 && g.bsy0 <= g.detysize && g.bsz0 <= g.bsz1 && g.bsz1 >= 1.0 &&
+                  g.bsz0 <= g.detzsize;
     g.dety0f = (float)g.dety0;
     g.detz0f = (float)g.detz0;
     g.rpxyf = (float)(1.0 / g.pxy);
@@ -374,14 +380,14 @@ int run_score(grc_ctx *ctx, const grc::Work &w, int64_t n_trials, bool comp = fa
             fused_key = true;
         }
         const int mode = comp ? grc::kScanComp : grc::kScanFull;
-        // Full output over more than two scan rounds goes to the CTA sweep: its CTAs walk each
-        // projection window in step and share the gathered 8-bit codes in L2 (FCC Al 2048^2 x 361,
-        // 64 seeds x 32,768 orientations per call: 16.1 M trials/s against 13.5 M on the warp
-        // scan).  Completeness-only calls and calls of one or two rounds take the warp scan (one
-        // seed, full output: 15.9 against 15.3 M trials/s end to end; 64 seeds, completeness
-        // only: 19.7 against 17.4 M).
+        // Trials of few pairs leave the warp scan's 32-projection spans and per-trial tables little
+        // to share: below 5,000 (projection, reflection) pairs the CTA sweep takes full-output calls
+        // of more than two rounds (90,000 trials, FCC Al: 0.98 against 1.04 ms at 37 x 64 pairs, 1.50
+        // against 1.46 at 73 x 64, 3.20 against 2.77 at 181 x 64, 32.6 against 25.4 for 524,288 at
+        // 361 x 64 on 2048^2).  Everything else, and all completeness-only calls, the warp scan.
+        const bool few_pairs = (int64_t)ctx->geo.nrot * ctx->geo.nhkl < 5000;
         const bool sweep = ctx->force_path == 2 ||
-                           (ctx->force_path == 0 && !comp &&
+                           (ctx->force_path == 0 && !comp && few_pairs &&
                             n_trials > 2 * grc::scan_round_trials(ctx->geo, ctx->num_sms));
         if (sweep) {
             e = grc::launch_sweep(ctx->geo, b, w, n_trials, ctx->num_sms, ctx->stream, e0, e1, &launches, 0, mode);

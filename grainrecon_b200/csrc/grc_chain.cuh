@@ -56,15 +56,15 @@ __device__ __forceinline__ OmegaRow omega_row(const Geo &g, const double2 cs, co
     const double c = cs.x, s = cs.y;
     const double swx = c * spx - s * spy, swy = s * spx + c * spy, swz = spz;
     const double gx = g.lss + swx, gy = swy - g.p0y + g.rao, gz = swz - g.p0z;
-    const double ngp = sqrt(gx * gx + gy * gy + gz * gz);
+    const double n2 = gx * gx + gy * gy + gz * gz, rn = rsqrt(n2), rx = 1.0 / gx;
     OmegaRow r;
-    r.kx = gx / ngp;
-    r.ky = gy / ngp;
-    r.kz = gz / ngp;
-    r.L2 = (g.lsd - swx) * ngp / gx;  // (Lsd - SamposW_x) / cos(alpha)
+    r.kx = gx * rn;
+    r.ky = gy * rn;
+    r.kz = gz * rn;
+    r.L2 = (g.lsd - swx) * (n2 * rn) * rx;  // (Lsd - SamposW_x) / cos(alpha)
     r.ax = g.lsd - swx;
-    r.ay = gy * L / gx - swy;
-    r.az = gz * L / gx - swz;
+    r.ay = gy * L * rx - swy;
+    r.az = gz * L * rx - swz;
     const double dx = swx - g.lsd, dy = swy - g.dety00 + g.rao, dz = swz - g.detz00;
     r.num = -(g.R[0] * dx + g.R[3] * dy + g.R[6] * dz);
     r.r2d = g.R[1] * dx + g.R[4] * dy + g.R[7] * dz;
@@ -79,15 +79,15 @@ __device__ __forceinline__ RowF row_f32(const Geo &g, const OmegaRow &r) {
     RowF f;
     f.cN = (float)(g.R[0] * r.ax);
     f.ky = (float)r.ky; f.kz = (float)r.kz; f.L2 = (float)r.L2;
-    f.cY = (float)(g.R[1] * r.ax / g.pxy);
+    f.cY = (float)(g.R[1] * r.ax * g.rpxy);
     f.ay = (float)r.ay; f.az = (float)r.az; f.num = (float)r.num;
-    f.u0 = (float)(g.dety0 - r.r2d / g.pxy);
-    f.v0 = (float)(g.detz0 - r.r3d / g.pxz);
+    f.u0 = (float)(g.dety0 - r.r2d * g.rpxy);
+    f.v0 = (float)(g.detz0 - r.r3d * g.rpxz);
     f.c = (float)r.c; f.s = (float)r.s;
     f.wx = (float)(r.c * r.kx + r.s * r.ky);
     f.wy = (float)(-r.s * r.kx + r.c * r.ky);
     f.wz = (float)r.kz;
-    f.cZ = (float)(g.R[2] * r.ax / g.pxz);
+    f.cZ = (float)(g.R[2] * r.ax * g.rpxz);
     return f;
 }
 
@@ -139,16 +139,17 @@ __device__ void build_gw(const Geo &g, const double *__restrict__ hkl, const dou
 // expanded, and the ray/plane intersection without normalising K_out.
 __device__ __forceinline__ int64_t landing_fp64(const Geo &g, const OmegaRow &r, double gxw, double gyw,
                                                 double gzw, int iw, double *lam_out = nullptr) {
-    const double G = sqrt(gxw * gxw + gyw * gyw + gzw * gzw);
+    // one reciprocal (square root) per length: an FP64 division or square root is some 25 instructions
+    const double rG = rsqrt(gxw * gxw + gyw * gyw + gzw * gzw);
     const double Gtx = r.c * gxw - r.s * gyw, Gty = r.s * gxw + r.c * gyw, Gtz = gzw;
-    const double x = (r.kx * Gtx + r.ky * Gty + r.kz * Gtz) / G;  // cos(beta)
-    const double lam = 2.0 * (2.0 * CUDART_PI / G) * (-x);        // 2 d sin(theta)
+    const double x = (r.kx * Gtx + r.ky * Gty + r.kz * Gtz) * rG;  // cos(beta)
+    const double lam = 2.0 * (2.0 * CUDART_PI * rG) * (-x);        // 2 d sin(theta)
     if (lam_out) *lam_out = lam;
     if (!(x < 0.0 && x > g.cbmax && lam > g.lmin && lam < g.lmax)) return -1;
     const double st = -x, ct = sqrt(1.0 - x * x);
     const double s2 = 2.0 * st * ct, c2 = 1.0 - 2.0 * st * st;
-    const double konst = sqrt(Gty * Gty + Gtz * Gtz);
-    const double gy = Gty / konst, gz = Gtz / konst;
+    const double rk = rsqrt(Gty * Gty + Gtz * Gtz);
+    const double gy = Gty * rk, gz = Gtz * rk;
     const double cphx = gy * r.ky + gz * r.kz;
     const double sphx = sqrt(fmax(0.0, 1.0 - cphx * cphx));
     const double sphy = sphx * c2 - cphx * s2;
@@ -158,7 +159,7 @@ __device__ __forceinline__ int64_t landing_fp64(const Geo &g, const OmegaRow &r,
     const double f = r.num / nK;
     const double y2 = f * (g.R[1] * Kx + g.R[4] * Ky + g.R[7] * Kz) + r.r2d;
     const double z2 = f * (g.R[2] * Kx + g.R[5] * Ky + g.R[8] * Kz) + r.r3d;
-    const double u = g.dety0 - y2 / g.pxy, v = g.detz0 - z2 / g.pxz;
+    const double u = g.dety0 - y2 * g.rpxy, v = g.detz0 - z2 * g.rpxz;
     // 1 <= round(u) <= detysize  <=>  0.5 <= u < detysize + 0.5 (round half away from zero)
     if (!(u >= 0.5 && u < g.detysize + 0.5 && v >= 0.5 && v < g.detzsize + 0.5)) return -1;
     const double ru = round(u), rv = round(v);
@@ -192,6 +193,41 @@ __device__ __forceinline__ float4 window_of(const Geo &g, float G_f) {
     lo = fmax(lo, 0.0);
     const double m = 1e-5 * G;  // >> FP32 error of k_w . G (~4e-7 |G|)
     return make_float4((float)(lo - m), (float)(hi + m), (float)(lo + m), (float)(hi - m));
+}
+
+// MUFU reciprocal and reciprocal square root without the denormal scaling code around them: every
+// argument here is a normal number (|G|, sines of window angles, lengths in mm) except in degenerate
+// landings, where 0 or a denormal gives Inf / NaN and the item goes to the exact path.
+__device__ __forceinline__ float rsq_approx(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// In-plane map offset of an FP32 landing (u, v): (dety-1)*detzsize + (detz-1), -1 for a certain
+// rejection, or -2 within the ambiguity band of a pixel edge or when `certain` is false.  Selects
+// instead of branches: the lanes of a batch part at every test.
+__device__ __forceinline__ int pixel_of(const Geo &g, float u, float v, bool certain) {
+    // nearest integer by the 1.5*2^23 addition: for |u| < 2^22 the sum's low mantissa bits hold the
+    // rounded value, read back as an integer without a conversion instruction.  Within the
+    // ambiguity band of a half-pixel the item goes to the exact path, so the tie rule of the
+    // rounding never decides anything; NaN and Inf fail the band test too.  A finite value of 2^22
+    // and more leaves an integer outside 1..10^6 (detectors have at most 10^6 pixels per side), a
+    // certain rejection.
+    constexpr float kRound = 12582912.0f;
+    const float tu = __fadd_rn(u, kRound), tv = __fadd_rn(v, kRound);
+    const float ru = __fsub_rn(tu, kRound), rv = __fsub_rn(tv, kRound);
+    certain = certain & (fabsf(u - ru) <= 0.5f - kAmbigPx) & (fabsf(v - rv) <= 0.5f - kAmbigPx);
+    const uint32_t iu = (uint32_t)(__float_as_int(tu) - 0x4B400001), iv = (uint32_t)(__float_as_int(tv) - 0x4B400001);
+    bool in = (iu < (uint32_t)g.detysize) & (iv < (uint32_t)g.detzsize);  // 0-based pixel
+    if (g.beam_stop) in = in & !((ru >= g.bsy0f) & (ru <= g.bsy1f) & (rv >= g.bsz0f) & (rv <= g.bsz1f));
+    const int ip = (int)(iu * (uint32_t)g.detzsize + iv);  // < 2^31 pixels per plane
+    return certain ? (in ? ip : -1) : -2;
 }
 
 // FP32 landing chain (the algebra of landing_fp64 with the row's constant terms folded in).
@@ -240,12 +276,37 @@ __device__ __forceinline__ int landing_fp32(const Geo &g, const RowF &r, const f
     return (int)((uint32_t)(iu - 1) * (uint32_t)g.detzsize + (uint32_t)(iv - 1));  // < 2^31 pixels per plane
 }
 
+// The same landing from a row of 12 numbers, {kx, ky, kz, L2}, {cN, ay, az, num}, {u0, v0, c, s}: cY
+// and cZ are multiples of cN, and k_in . (Omega Gw) is formed with the rotated G, so a lane reads
+// three 16-byte words of its projection instead of four.  A radicand below zero by rounding (x or
+// cphx beyond 1) gives NaN, so the exact path decides.
+__device__ __forceinline__ int landing_row3(const Geo &g, const float4 k, const float4 a, const float4 o,
+                                            const float4 gw, float lo_in, float hi_in) {
+    const float Gtx = o.z * gw.x - o.w * gw.y, Gty = o.w * gw.x + o.z * gw.y, Gtz = gw.z;
+    const float dot = k.x * Gtx + k.y * Gty + k.z * Gtz;
+    const bool inside = (-dot > lo_in) & (-dot < hi_in);
+    const float x = dot * gw.w, x2 = x * x;
+    const float q = 1.0f - x2, c2 = 1.0f - 2.0f * x2;
+    const float s2 = (-2.0f * x) * (q * rsq_approx(q));
+    const float rk = rsq_approx(Gty * Gty + Gtz * Gtz);
+    const float gy = Gty * rk, gz = Gtz * rk;
+    const float cphx = gy * k.y + gz * k.z;
+    const float p = 1.0f - cphx * cphx;
+    const float sphy = (p * rsq_approx(p)) * c2 - cphx * s2;
+    const float diff = (k.w * s2) * rcp_approx(sphy);
+    const float Ky = a.y + diff * gy, Kz = a.z + diff * gz;
+    const float f = a.w * rcp_approx(a.x + g.Rf[3] * Ky + g.Rf[6] * Kz);
+    const float u = o.x - f * (g.Raf[0] * a.x + (g.Ruf[0] * Ky + g.Ruf[1] * Kz));
+    const float v = o.y - f * (g.Raf[1] * a.x + (g.Rvf[0] * Ky + g.Rvf[1] * Kz));
+    return pixel_of(g, u, v, inside);
+}
+
 // Gw (FP32) of one reflection from the slot's S*U*B and h; .w = 1/|Gw|.
 __device__ __forceinline__ float4 gw_of(const float *sf, const float4 h) {
     const float x = sf[0] * h.x + sf[1] * h.y + sf[2] * h.z;
     const float y = sf[3] * h.x + sf[4] * h.y + sf[5] * h.z;
     const float z = sf[6] * h.x + sf[7] * h.y + sf[8] * h.z;
-    return make_float4(x, y, z, rsqrtf(x * x + y * y + z * z));
+    return make_float4(x, y, z, rsq_approx(x * x + y * y + z * z));
 }
 
 // Window on t = -(k_w . Gw) in FP32 (see window_of) from rG = 1/|G|; the 1e-5 |G|

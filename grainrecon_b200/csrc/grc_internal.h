@@ -19,6 +19,7 @@ constexpr int kFallbackCap = 64;       // ambiguous items awaiting the FP64 path
 struct Geo {
     double lss, lsd, p0y, p0z, dety00, detz00, pxy, pxz, rao;
     double dety0, detz0;
+    double rpxy, rpxz;       // 1 / pixel sizes
     double lmin, lmax;       // wavelength window [A]
     double cbmax;            // cos((90+4*thetamax) deg), or -2 when that angle is >= 180 deg
     double bsy0, bsy1, bsz0, bsz1;
@@ -26,8 +27,10 @@ struct Geo {
     // FP32 copies for the fast landing chain
     float Rf[9];
     float Ruf[2], Rvf[2];    // R[4]/pxy, R[7]/pxy and R[5]/pxz, R[8]/pxz (ray K -> pixel u, v)
+    float Raf[2];            // R[1]/(R[0] pxy) and R[2]/(R[0] pxz) (the same for R[0] K_x)
     float dety0f, detz0f, rpxyf, rpxzf;
     float bsy0f, bsy1f, bsz0f, bsz1f;
+    int beam_stop;           // 0 when the beam stop covers no pixel of the detector
     float lo4pif, hi4pif, cbmaxf;   // lambda_min/(4 pi), lambda_max/(4 pi), cos(beta_max)
     int nhkl, nrot, detysize, detzsize;
     uint32_t n_hit;          // codes [0, n_hit) are "dis <= threshold"

@@ -4,19 +4,30 @@
 // every CTA walking the projections window by window so the map pixels being read stay in L2),
 // organised around the warp instead of the CTA:
 //   * a warp takes one trial (slot) of the window at a time and first writes that trial's FP32
-//     Gw table and window thresholds for all reflections into its own shared-memory table; the
-//     prefilter keeps them in registers (lanes on reflections, as the sweep) and the per-item
-//     landing reads them from the table instead of recomputing S*U*B*h and the window;
-//   * the survivors of a trial go through a per-warp queue, 32 at a time, through the FP32 landing
-//     chain with its FP64 band (landing_fp32 / landing_exact), and the queue is emptied at the end
-//     of the trial, so every batch belongs to one trial: its pixels are counted in one register
-//     of the warp (completeness-only mode: one bit of the packed hit mask per pixel) or in the
-//     trial's 8-bit code histogram (full mode: Nr_simu, Nr_intersect and the exact median).
-// Ambiguous items keep their trial in the FP64 queue, which is drained at the end of the window.
+//     Gw table and window thresholds for all reflections into its own shared-memory table;
+//   * 32 projections at a time, each lane tests its reflections against the window and shifts the
+//     sign of the test into a bit mask (6 instructions per pair, no ballot, no store); the set
+//     bits of a mask are runs of consecutive projections, and one entry and one mark bit per run
+//     number the passing pairs, so that a batch of 32 finds its pairs by a population count;
+//   * batches go through the FP32 landing chain with its FP64 band (landing_row3 / landing_exact).
+//     Lanes hold consecutive projections of a few reflections: their omega rows are consecutive
+//     16-byte words in shared memory, their Gw words broadcasts;
+//   * a selected pixel's map word is read when its batch is evaluated and counted some batches
+//     later: two, in registers, for the bit mask; three, through cp.async, for the 8-bit codes, of
+//     which a third miss L2;
+//   * ambiguous items keep their trial in the warp's FP64 queue, drained outside the batch loop: a
+//     call inside it cost 12 spill reloads per batch.
+// What bounds it (FCC Al 2048^2 x 361, completeness): issue (69 % of slots, 28.3 k warp instructions
+// per trial) and the shared-memory / L1 pipe (78 % of its wavefronts: 12 of a batch's 56 are its
+// rows, some 20 its gather) together.  Against one ballot and one queue store per (projection, slot)
+// and 64-byte rows (40.6 k instructions): 64 seeds x 32,768 orientations 97.4 -> 73.2 ms, four
+// columns (16 seeds) 32.6 (CTA sweep) -> 25.6 ms.  Numbering the pairs projection-major instead
+// (masks transposed across the warp, better shared rows) ran 82.0 ms: its Gw words conflict.  Four
+// CTAs per SM (64 registers) ran 114 ms.
 // Windows: up to 32 projections of 8-bit codes (full mode), up to 128 of the bit mask
 // (completeness mode), each within the limits of shared memory and L2 (launch_scan_t).
 // The decisions are those of the sweep and of the oracle: same prefilter margins, same FP32
-// chain and band, same FP64 path.
+// algebra and band, same FP64 path.
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <stdint.h>
@@ -48,8 +59,18 @@ __device__ __forceinline__ int64_t scan_orient_of(const Work &w, int64_t t, int6
     return w.diag ? t : (t - v * w.n_or);
 }
 
+// Omega row of one (voxel, projection) as four float4 planes of WIN projections each, so that lanes
+// on consecutive projections read consecutive 16-byte words: {kx, ky, kz, L2}, {cN, ay, az, num},
+// {u0, v0, c, s} for the landing and {wx, wy, wz, -} = k_w for the window test.
+constexpr int kRowParts = 4;
+// Landings of a (trial, window) awaiting their batch: fewer than 64 left over plus one run of up to
+// 32 projections per lane, one mark bit each, in rings.
+constexpr int kMarkRing = 64;  // words of 32 positions
+constexpr int kRunRing = 128;
+constexpr int kStages = 4;     // full mode: batches whose map words are in flight
+
 struct ScanSmem {
-    RowF *rows;        // [rows_cap * nwin] omega rows of the window, vloc * nwin + wl
+    float4 *rows;      // [rows_cap][kRowParts][nwin] omega rows of the window
     float4 *hk;        // [nhkl] h as float
     uint32_t *hist;    // full mode: [slots * kHistWords]; completeness mode: [slots] packed counters
     float *subf;       // [slots * 12]
@@ -57,13 +78,20 @@ struct ScanSmem {
     int *vloc;         // [slots]
     int64_t *vglob;    // [slots]
     int64_t *vlist;    // [slots]
-    float4 *wgw;       // [kWarps * nhkl] per-warp Gw table of the warp's trial: x, y, z, 1/|G|
-    float4 *wwin;      // [kWarps * nhkl] its window thresholds (window_f)
-    uint32_t *queue;   // [kWarps * kQueueCap]
-    uint32_t *fqueue;  // [kWarps * kFallbackCap]
+    unsigned char *warps;  // [kWarps] blocks of warp_block_bytes(nhkl)
 };
 
-constexpr int kScanParts = 11;
+// A warp's own block: rings, queues and the tables of its trial at fixed offsets from one base.
+constexpr int kExactCap = 128;                              // ambiguous items awaiting the FP64 path
+constexpr int kOffRuns = kMarkRing * 4;                     // [kRunRing]
+constexpr int kOffExact = kOffRuns + kRunRing * 4;          // [kExactCap]
+constexpr int kOffTable = kOffExact + kExactCap * 4;        // [nhkl] {Gw x, y, z, 1/|G|}, {certain lo, hi, middle, half}
+// ... and in full mode after it [kStages * 32] map words of the batches in flight
+__host__ __device__ inline size_t warp_block_bytes(int mode, int nhkl) {
+    return kOffTable + sizeof(float4) * 2 * nhkl + (mode == kScanFull ? sizeof(uint32_t) * kStages * 32 : 0);
+}
+
+constexpr int kScanParts = 9;
 __host__ __device__ inline size_t scan_smem_layout(int mode, int nhkl, int rows_cap, int slots, int nwin,
                                                    size_t *offs) {
     size_t o = 0, i = 0;
@@ -72,7 +100,7 @@ __host__ __device__ inline size_t scan_smem_layout(int mode, int nhkl, int rows_
         offs[i++] = o;
         o += bytes;
     };
-    put(sizeof(RowF) * rows_cap * nwin);
+    put(sizeof(float4) * kRowParts * rows_cap * nwin);
     put(sizeof(float4) * nhkl);
     put(sizeof(uint32_t) * slots * (mode == kScanFull ? kHistWords : 1));
     put(sizeof(float) * slots * 12);
@@ -80,21 +108,26 @@ __host__ __device__ inline size_t scan_smem_layout(int mode, int nhkl, int rows_
     put(sizeof(int) * slots);
     put(sizeof(int64_t) * slots);
     put(sizeof(int64_t) * slots);
-    put(sizeof(float4) * kWarps * nhkl);
-    put(sizeof(float4) * kWarps * nhkl);
-    put(sizeof(uint32_t) * kWarps * kQueueCap);
-    o = (o + 15) & ~size_t(15);
-    offs[i] = o;  // fqueue
-    o += sizeof(uint32_t) * kWarps * kFallbackCap;
+    put(kWarps * warp_block_bytes(mode, nhkl));
     return (o + 15) & ~size_t(15);
+}
+
+__device__ __forceinline__ void cp_async4(uint32_t *dst, const uint32_t *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
 __device__ __forceinline__ ScanSmem scan_carve(unsigned char *base, int mode, int nhkl, int rows_cap, int slots,
                                                int nwin) {
-    size_t offs[kScanParts + 1];
+    size_t offs[kScanParts];
     scan_smem_layout(mode, nhkl, rows_cap, slots, nwin, offs);
     ScanSmem m;
-    m.rows = (RowF *)(base + offs[0]);
+    m.rows = (float4 *)(base + offs[0]);
     m.hk = (float4 *)(base + offs[1]);
     m.hist = (uint32_t *)(base + offs[2]);
     m.subf = (float *)(base + offs[3]);
@@ -102,10 +135,7 @@ __device__ __forceinline__ ScanSmem scan_carve(unsigned char *base, int mode, in
     m.vloc = (int *)(base + offs[5]);
     m.vglob = (int64_t *)(base + offs[6]);
     m.vlist = (int64_t *)(base + offs[7]);
-    m.wgw = (float4 *)(base + offs[8]);
-    m.wwin = (float4 *)(base + offs[9]);
-    m.queue = (uint32_t *)(base + offs[10]);
-    m.fqueue = (uint32_t *)(base + offs[11]);
+    m.warps = base + offs[8];
     return m;
 }
 
@@ -119,11 +149,11 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
     const ScanSmem sm = scan_carve(smem_raw, MODE, g.nhkl, rows_cap, slots, WIN);
     __shared__ int s_nv, s_next;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const unsigned lt = (1u << lane) - 1u;
-    uint32_t *wq = sm.queue + warp * kQueueCap;
-    uint32_t *fq = sm.fqueue + warp * kFallbackCap;
-    float4 *gwt = sm.wgw + warp * g.nhkl;
-    float4 *wnt = sm.wwin + warp * g.nhkl;
+    const unsigned lt = (1u << lane) - 1u, le = lt | (1u << lane);
+    unsigned char *wb = sm.warps + warp * warp_block_bytes(MODE, g.nhkl);
+    uint32_t *marks = (uint32_t *)wb, *runs = (uint32_t *)(wb + kOffRuns), *fq = (uint32_t *)(wb + kOffExact);
+    float4 *tab = (float4 *)(wb + kOffTable);
+    uint32_t *stage = (uint32_t *)(tab + 2 * g.nhkl) + lane;  // full mode
 
     // ---- set-up: per-slot S*U*B, voxels, zeroed counters
     if (tid < nslot) {
@@ -142,6 +172,7 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
     for (int i = tid; i < slots * (MODE == kScanFull ? kHistWords : 1); i += kThreads) sm.hist[i] = 0;
     for (int i = tid; i < g.nhkl; i += kThreads)
         sm.hk[i] = make_float4((float)b.hkl[3 * i], (float)b.hkl[3 * i + 1], (float)b.hkl[3 * i + 2], 0.f);
+    for (int i = lane; i < kMarkRing; i += 32) marks[i] = 0;
     __syncthreads();
     if (tid == 0) {
         int nv = 0;
@@ -161,13 +192,33 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
         // ---- omega rows of this window for every voxel of the round
         for (int i = tid; i < nv * nw; i += kThreads) {
             const int vl = i / nw, wl = i - vl * nw;
-            sm.rows[vl * WIN + wl] = row_f32(g, omega_row(g, b.rot_cs[w0 + wl], b.vpos + 3 * sm.vlist[vl]));
+            const OmegaRow d = omega_row(g, b.rot_cs[w0 + wl], b.vpos + 3 * sm.vlist[vl]);
+            const RowF r = row_f32(g, d);
+            float4 *o = sm.rows + vl * kRowParts * WIN + wl;
+            o[0] = make_float4((float)d.kx, r.ky, r.kz, r.L2);
+            o[WIN] = make_float4(r.cN, r.ay, r.az, r.num);
+            o[2 * WIN] = make_float4(r.u0, r.v0, r.c, r.s);
+            o[3 * WIN] = make_float4(r.wx, r.wy, r.wz, 0.f);
         }
         if (tid == 0) s_next = 0;
         __syncthreads();
 
+        // the window's 8-bit codes as 32-bit words; its first pixel may start inside a word, at byte wmis
         const uint8_t *wcodes = MODE == kScanFull ? b.codes8 + (int64_t)w0 * g.plane : nullptr;
+        const uint32_t wmis = (uint32_t)((uintptr_t)wcodes & 3u);
+        const uint32_t *wwords = (const uint32_t *)(wcodes - wmis);
         const uint32_t *wbits = MODE == kScanComp ? b.bits + (int64_t)w0 * pw : nullptr;
+        // Full mode: the map word of a selected pixel is copied to shared memory when its batch is
+        // evaluated and its code counted kStages - 1 batches later, whichever trials those belong
+        // to, so the gather's latency (a third of the codes miss L2) overlaps their landings.  A byte
+        // per batch in flight: 0x80 | bit of the code in its word, or 0; and the batch's trial.
+        uint32_t pend = 0, pend_slot = 0;
+        int n_batch = 0;
+        auto count_oldest = [&]() {
+            if (!(pend & 0x80000000u)) return;
+            const uint32_t code = (stage[(n_batch & (kStages - 1)) * 32] >> ((pend >> 24) & 31u)) & 255u;
+            atomicAdd(&sm.hist[(pend_slot >> 24) * kHistWords + (code >> 1)], 1u << ((code & 1u) * 16));
+        };
         int fn = 0;  // ambiguous items of this warp (any of its trials), drained at the window end
 
         // FP64 path of one ambiguous item: counted at once (shared atomics; these items are rare)
@@ -205,108 +256,201 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
             if (lane == 0) s = atomicAdd(&s_next, 1);
             s = __shfl_sync(kAll, s, 0);
             if (s >= nslot) break;
+            // ---- the trial's Gw and window table
             const float *sf = sm.subf + 12 * s;
-            // ---- the trial's Gw table (shared, for the landings) and prefilter (registers)
-            float gx[HPL], gy[HPL], gz[HPL], lo[HPL], hi[HPL];
 #pragma unroll
             for (int j = 0; j < HPL; ++j) {
                 const int ih = lane + 32 * j;
-                gx[j] = gy[j] = gz[j] = 0.f;
-                lo[j] = CUDART_INF_F;
-                hi[j] = -CUDART_INF_F;
                 if (ih < g.nhkl) {
                     const float4 gv = gw_of(sf, sm.hk[ih]);
                     const float4 wv = window_f(g, gv);
-                    gwt[ih] = gv;
-                    wnt[ih] = wv;
-                    gx[j] = gv.x;
-                    gy[j] = gv.y;
-                    gz[j] = gv.z;
-                    lo[j] = wv.x;
-                    hi[j] = wv.y;
+                    tab[2 * ih] = gv;
+                    tab[2 * ih + 1] = make_float4(wv.z, wv.w, 0.5f * (wv.x + wv.y), 0.5f * (wv.y - wv.x));
                 }
             }
             __syncwarp();
-            const RowF *vr = sm.rows + sm.vloc[s] * WIN;
+            const float4 *vr = sm.rows + sm.vloc[s] * kRowParts * WIN;
             // completeness mode: the lane's share of this trial's counts in this window, packed as
             // the shared counter (Nr_simu low, Nr_intersect high 16 bits) and summed over the warp
             // once per trial and window
             uint32_t cnt = 0;
-            // a selected pixel is read when its batch is evaluated and counted after the next batch
-            // has been computed, so the gather's latency overlaps the landing arithmetic; pend_bit
-            // is the pixel's bit (completeness) or 0 (full), -1 when the lane has none
-            int pend_bit = -1;
-            uint32_t pend_val = 0;
-            auto apply_pending = [&]() {
-                if (MODE == kScanComp) {
-                    const bool sel = pend_bit >= 0;
-                    const bool hit = sel && ((pend_val >> pend_bit) & 1u);
-                    cnt += (uint32_t)sel + ((uint32_t)hit << 16);
-                } else if (pend_bit >= 0) {
-                    atomicAdd(&sm.hist[s * kHistWords + (pend_val >> 1)], 1u << ((pend_val & 1u) * 16));
-                }
-                pend_bit = -1;
-            };
-            auto fast = [&](uint32_t item, bool valid) {
-                const int wl = (int)(item >> 8), ih = (int)(item & 255u);
+            // Completeness mode: a selected pixel's map word is read when its batch is evaluated and
+            // counted after the next two batches have been computed, so the gather's latency overlaps
+            // the landing arithmetic (pend_bit: the pixel's bit in the word)
+            int pend_bit[2] = {0, 0};
+            uint32_t pend_word[2] = {0, 0};
+            // Positions 0, 1, 2, ... number the trial's (reflection, projection) pairs that pass the
+            // window test, one run of consecutive projections of a reflection after the other.  A
+            // mark bit says where a run starts, and its entry holds the reflection and the projection
+            // minus the position, so a lane finds its pair from a population count.
+            int end = 0, done = 0;      // positions known / evaluated (done: a multiple of 64)
+            int n_run = 0, r_run = -1;  // runs known / index of the run that position `done` lies in
+            // the pair at position `pos`; h: the pending pixel it takes the place of (constant)
+            auto one = [&](int h, uint32_t e, int pos, bool valid) {
+                const int ih = (int)(e & 255u), wl = ((int)e >> 8) + pos;
                 int ip = -1;
                 if (valid) {
-                    const float4 gv = gwt[ih];
-                    const float4 wv = wnt[ih];
-                    ip = landing_fp32(g, vr[wl], gv, wv.z, wv.w);
+                    const float4 gv = tab[2 * ih];
+                    const float2 wv = *(const float2 *)(tab + 2 * ih + 1);
+                    const float4 *o = vr + wl;
+                    ip = landing_row3(g, o[0], o[WIN], o[2 * WIN], gv, wv.x, wv.y);
                 }
+#ifdef GRC_AUDIT
+                // audit build: every certain FP32 decision is re-decided by the FP64 path
+                if (valid && ip != -2) {
+                    const int64_t r64 = landing_exact(b.geo, b.rot_cs, b.vpos + 3 * sm.vglob[s], b.hkl,
+                                                      sm.subd + 9 * s, w0 + wl, ih);
+                    atomicAdd((unsigned long long *)(b.work_counter + 6), 1ull);
+                    if ((r64 >= 0 ? (int)(r64 - (int64_t)(w0 + wl) * g.plane) : -1) != ip)
+                        atomicAdd(b.work_counter + 5, 1);
+                }
+#endif
                 const unsigned m = __ballot_sync(kAll, ip == -2);
+                // offsets within the window fit 32 bits: WIN * plane < 2^31 for the codes
+                // (launch_scan_t) and 8 * plane < 2^31 for the words (scan_round_trials)
+                if constexpr (MODE == kScanComp) {
+                    uint32_t word = 0;
+                    if (ip >= 0) {
+                        word = __ldg(wbits + ((uint32_t)wl * pw32 + ((uint32_t)ip >> 5)));
+                        cnt += 1u;
+                    }
+                    cnt += ((pend_word[h] >> pend_bit[h]) & 1u) << 16;
+                    pend_bit[h] = ip & 31;
+                    pend_word[h] = word;
+                } else {
+                    cp_async_wait<kStages - 1>();
+                    count_oldest();
+                    uint32_t info = 0;
+                    if (ip >= 0) {
+                        const uint32_t off = (uint32_t)wl * (uint32_t)g.plane + (uint32_t)ip + wmis;
+                        cp_async4(stage + (n_batch & (kStages - 1)) * 32, wwords + (off >> 2));
+                        info = 0x80u | (off & 3u) * 8u;
+                    }
+                    cp_async_commit();
+                    pend = (pend << 8) | info;
+                    pend_slot = (pend_slot << 8) | (uint32_t)s;
+                    ++n_batch;
+                }
                 if (m) {  // ambiguous items (rare) join the FP64 queue
-                    if (ip == -2) fq[fn + __popc(m & lt)] = ((uint32_t)s << 16) | item;
+                    if (ip == -2) fq[fn + __popc(m & lt)] = ((uint32_t)s << 16) | ((uint32_t)wl << 8) | (uint32_t)ih;
                     fn += __popc(m);
                 }
-                uint32_t val = 0;
-                if (ip >= 0) {
-                    // offsets within the window fit 32 bits: WIN * plane < 2^31 for the codes
-                    // (launch_scan_t) and 8 * plane < 2^31 for the words (scan_round_trials)
-                    if (MODE == kScanComp)
-                        val = __ldg(wbits + ((uint32_t)wl * pw32 + ((uint32_t)ip >> 5)));
-                    else
-                        val = __ldg(wcodes + ((uint32_t)wl * (uint32_t)g.plane + (uint32_t)ip));
-                }
-                apply_pending();
-                pend_bit = ip >= 0 ? (MODE == kScanComp ? (ip & 31) : 0) : -1;
-                pend_val = val;
             };
-            int qn = 0;
-            for (int wl = 0; wl < nw; ++wl) {
-                const float4 kwv = reinterpret_cast<const float4 *>(vr + wl)[3];
+            auto two_batches = [&](bool full) {
+                uint2 *mw = (uint2 *)(marks + ((done >> 5) & (kMarkRing - 1)));
+                const uint2 mm = *mw;
+                const int r1 = r_run + __popc(mm.x);
+                const uint32_t e0 = runs[(r_run + __popc(mm.x & le)) & (kRunRing - 1)];
+                const uint32_t e1 = runs[(r1 + __popc(mm.y & le)) & (kRunRing - 1)];
+                r_run = r1 + __popc(mm.y);
+                one(0, e0, done + lane, full || done + lane < end);
+                if (full || done + 32 < end) one(1, e1, done + 32 + lane, full || done + 32 + lane < end);
+                if (lane == 0) *mw = make_uint2(0, 0);  // every lane has read it: a ballot lies between
+                done += 64;
+            };
+            // ---- 32 projections at a time: the window test of every reflection as a bit mask per
+            // lane and slot, its runs of set bits numbered, full batches of 32 evaluated
+            constexpr int kSpan = WIN < 32 ? WIN : 32;
+            uint32_t rem[HPL];
+            bool tested = false;  // rem holds what is left of the span at k
+            int k = 0;
+            for (;;) {
+                // leaves this loop when the FP64 queue has no room for a batch, and comes back
+                while (k < nw) {
+                    if (!tested) {
+                        tested = true;
+                        float gx[HPL], gy[HPL], gz[HPL], mid[HPL], half[HPL];
 #pragma unroll
-                for (int j = 0; j < HPL; ++j) {
-                    const float t = -fmaf(kwv.x, gx[j], fmaf(kwv.y, gy[j], kwv.z * gz[j]));
-                    const bool pass = (t > lo[j]) && (t < hi[j]);
-                    const unsigned bm = __ballot_sync(kAll, pass);
-                    if (pass) wq[qn + __popc(bm & lt)] = ((uint32_t)wl << 8) | (uint32_t)(lane + 32 * j);
-                    qn += __popc(bm);
+                        for (int j = 0; j < HPL; ++j) {
+                            const int ih = lane + 32 * j;
+                            const bool real = ih < g.nhkl;
+                            const float4 gv = tab[real ? 2 * ih : 0];
+                            const float4 wv = tab[real ? 2 * ih + 1 : 1];
+                            gx[j] = gv.x;
+                            gy[j] = gv.y;
+                            gz[j] = gv.z;
+                            mid[j] = wv.z;
+                            half[j] = real ? wv.w : -1.0f;
+                            rem[j] = 0;
+                        }
+                        const float4 *kw = vr + 3 * WIN + k;
+#pragma unroll 8
+                        for (int p = kSpan - 1; p >= 0; --p) {
+                            const float4 q = kw[p];
+#pragma unroll
+                            for (int j = 0; j < HPL; ++j) {
+                                // |t - middle| - half is negative inside the window, t = -(k_w . Gw):
+                                // its sign bit joins the mask from below
+                                const float d = fmaf(q.x, gx[j], fmaf(q.y, gy[j], fmaf(q.z, gz[j], mid[j])));
+                                rem[j] = __funnelshift_l(__float_as_uint(fabsf(d) - half[j]), rem[j], 1);
+                            }
+                        }
+                        const uint32_t live = nw - k < 32 ? (1u << (nw - k)) - 1u : kAll;
+#pragma unroll
+                        for (int j = 0; j < HPL; ++j) rem[j] &= live;
+                    }
+                    bool spent = false;
+                    for (;;) {
+                        while (end - done >= 64 && fn <= kExactCap - 64) two_batches(true);
+                        if (end - done >= 64) break;
+                        // one run per lane: the first of its first slot that has any left
+                        uint32_t x = 0;
+                        int js = 0;
+#pragma unroll
+                        for (int j = HPL - 1; j >= 0; --j)
+                            if (rem[j]) x = rem[j], js = j;
+                        const unsigned any = __ballot_sync(kAll, x != 0);
+                        if (!any) {
+                            spent = true;
+                            break;
+                        }
+                        const uint32_t low = x & (0u - x), rest = x & (x + low);
+                        const int len = __popc(x ^ rest);
+#pragma unroll
+                        for (int j = 0; j < HPL; ++j)
+                            if (j == js) rem[j] = rest;
+                        int incl = len;
+#pragma unroll
+                        for (int o = 1; o < 32; o <<= 1) {
+                            const int y = __shfl_up_sync(kAll, incl, o);
+                            if (lane >= o) incl += y;
+                        }
+                        if (x) {
+                            const int pos = end + incl - len, first = k + 31 - __clz(low);
+                            runs[(n_run + __popc(any & lt)) & (kRunRing - 1)] =
+                                ((uint32_t)(first - pos) << 8) | (uint32_t)(lane + 32 * js);
+                            atomicOr(&marks[(pos >> 5) & (kMarkRing - 1)], 1u << (pos & 31));
+                        }
+                        end += __shfl_sync(kAll, incl, 31);
+                        n_run += __popc(any);
+                        __syncwarp();
+                    }
+                    if (!spent) break;
+                    tested = false;
+                    k += kSpan;
                 }
-                __syncwarp();
-                while (qn >= 32) {
-                    qn -= 32;
-                    const uint32_t item = wq[qn + lane];
-                    __syncwarp();
-                    fast(item, true);
-                    __syncwarp();
-                    drain_exact(false);
-                }
-            }
-            if (qn > 0) {  // the trial's last, partial batch: every batch holds one trial
-                const bool valid = lane < qn;
-                const uint32_t item = valid ? wq[lane] : 0u;
-                __syncwarp();
-                fast(item, valid);
+                if (k >= nw && fn <= kExactCap - 64) break;
                 __syncwarp();
                 drain_exact(false);
             }
-            apply_pending();
+            if (end > done) two_batches(false);  // the last ones: every batch holds one trial
+            __syncwarp();
             if (MODE == kScanComp) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h) cnt += ((pend_word[h] >> pend_bit[h]) & 1u) << 16;
 #pragma unroll
                 for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(kAll, cnt, o);
                 if (lane == 0) atomicAdd(&sm.hist[s], cnt);
+            }
+        }
+        if (MODE == kScanFull) {
+            cp_async_wait<0>();
+#pragma unroll
+            for (int i = 0; i < kStages; ++i) {  // the last batches, oldest first
+                count_oldest();
+                pend <<= 8;
+                pend_slot <<= 8;
+                ++n_batch;
             }
         }
         drain_exact(true);
@@ -337,12 +481,17 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
     }
 }
 
+// Shared memory that the CTAs of an SM may take together (1 KB reserved for each included).  Above
+// some 196 KB the SM is left with 28 KB of L1, and the misses in flight each need an L1 line: full-output
+// scans ran 12.9 ms with three CTAs of 24 to 40 trials and 19.4 ms with 48 to 64 (FCC Al 2048^2 x
+// 361, 8 seeds x 32,768 orientations), 5.43 against 6.96 ms on BCC Fe 1024^2 x 181.
+constexpr size_t kSmSmemBudget = 192 * 1024;
+
 template <int MODE, int HPL>
 cudaError_t launch_scan_t(const Geo &g, const ScoreBufs &b, const Work &w, int64_t n_trials, int num_sms,
                           cudaStream_t s, cudaEvent_t ev0, cudaEvent_t ev1, int *launches, int max_slots) {
-    // Tiles as the sweep: kScanSlotsBulk trials per CTA; an implicit seeding list may take up to
-    // kScanSlots when that fits the call into one round; explicit lists keep one row set per
-    // voxel-run start of their aligned 32-trial blocks.
+    // An implicit seeding list meets at most two voxels per tile; explicit lists keep one row set per
+    // voxel-run start of their aligned 32-trial blocks, or per trial when that bound is unknown.
     const bool explicit_voxels = w.trial_voxel || w.diag || w.n_or <= 0;
     const bool caller_tile = max_slots >= 1 && max_slots <= kScanSlots;
     if (!caller_tile) max_slots = kScanSlotsBulk;
@@ -351,46 +500,16 @@ cudaError_t launch_scan_t(const Geo &g, const ScoreBufs &b, const Work &w, int64
         if (explicit_voxels) rc = w.starts_per_32 > 0 ? 1 + ((sl + 31) / 32 + 1) * w.starts_per_32 : sl;
         return rc > sl ? sl : rc;
     };
-    size_t offs[kScanParts + 1];
+    size_t offs[kScanParts];
     using ScanFn = void (*)(Geo, ScoreBufs, Work, int64_t, int64_t, int, int);
-    const ScanFn k8 = scan_kernel<MODE, HPL, kScanWinMin>;
-    const size_t smem_max = scan_smem_layout(MODE, g.nhkl, rows_for(max_slots), max_slots, kScanWinMin, offs);
-    int per_sm = 0;
-    cudaError_t e = occupancy_for((const void *)k8, smem_max, &per_sm);
-    if (e != cudaSuccess) return e;
-    if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    const int64_t grid = (int64_t)per_sm * num_sms;
-    if (!caller_tile && !explicit_voxels && n_trials > grid * max_slots && n_trials <= grid * kScanSlots) {
-        int per_sm1 = 0;
-        const size_t smem1 = scan_smem_layout(MODE, g.nhkl, rows_for(kScanSlots), kScanSlots, kScanWinMin, offs);
-        if (occupancy_for((const void *)k8, smem1, &per_sm1) == cudaSuccess && per_sm1 == per_sm)
-            max_slots = kScanSlots;
-    }
-    const int64_t rounds = (n_trials + grid * max_slots - 1) / (grid * max_slots);
-    int slots = (int)((n_trials + rounds * grid - 1) / (rounds * grid));
-    if (slots < 1) slots = 1;
-    const int rows_cap = rows_for(slots);
-    // the widest projection window whose rows keep the grid's CTAs per SM: up to 128 projections
-    // for the bit mask of a seeding scan (one-seed Al rounds 1.641 / 1.567 / 1.573 ms at 32 / 64 /
-    // 128, 64-seed calls 103.9 / 98.7 / 97.1 ms), 32 or 16 for the 8-bit codes (32 projections of
-    // 2048^2 codes are already about the size of L2; 16 ran 6-8 % slower), else 8
-    ScanFn kern = k8;
-    size_t smem = scan_smem_layout(MODE, g.nhkl, rows_cap, slots, kScanWinMin, offs);
-    bool refused = false;
-    auto window_kernel = [](int cand) -> ScanFn {
+    auto window_kernel = [](int win) -> ScanFn {
         if constexpr (MODE == kScanComp) {
-            if (cand == 128) return scan_kernel<MODE, HPL, 128>;
-            if (cand == 64) return scan_kernel<MODE, HPL, 64>;
+            if (win == 128) return scan_kernel<MODE, HPL, 128>;
+            if (win == 64) return scan_kernel<MODE, HPL, 64>;
         }
-        return cand == 32 ? (ScanFn)scan_kernel<MODE, HPL, 32> : (ScanFn)scan_kernel<MODE, HPL, 16>;
+        if (win == 32) return scan_kernel<MODE, HPL, 32>;
+        return win == 16 ? (ScanFn)scan_kernel<MODE, HPL, 16> : (ScanFn)scan_kernel<MODE, HPL, kScanWinMin>;
     };
-    // Explicit trial lists in completeness mode (the seeding refine's grids) take at most 64: the
-    // refine of 16 Al seeds took 0.223 s with 64-projection windows, 0.234 s with 32 and
-    // 0.246-0.255 s with 128.
-    const bool wide = MODE == kScanComp;
-    const int kCands = wide ? 4 : 2;
-    const int cands_wide[4] = {explicit_voxels ? 64 : 128, 64, 32, 16}, cands_narrow[2] = {32, 16};
-    const int *cands = wide ? cands_wide : cands_narrow;
     // the bit-mask window stays within 3/4 of L2 (Al 2048^2 on 126 MB: 128 projections = 67 MB,
     // fastest; 256 = 134 MB ran 30% slower)
     int64_t l2_budget = 0;
@@ -401,24 +520,50 @@ cudaError_t launch_scan_t(const Geo &g, const ScoreBufs &b, const Work &w, int64
         else
             cudaGetLastError();  // no L2 size: windows of at most 32 projections
     }
-    for (int ci = 0; ci < kCands; ++ci) {
-        const int cand = cands[ci];
-        if (MODE == kScanComp && cand > 32 && (int64_t)cand * b.plane_words * 4 > l2_budget) continue;
-        if (MODE == kScanFull && (int64_t)cand * g.plane > 2147483647LL) continue;
-        const ScanFn kc = window_kernel(cand);
-        const size_t smem_c = scan_smem_layout(MODE, g.nhkl, rows_cap, slots, cand, offs);
-        int per_c = 0;
-        if (occupancy_for((const void *)kc, smem_c, &per_c) != cudaSuccess) {
-            refused = true;
-            continue;
-        }
-        if (per_c >= per_sm) {
-            kern = kc;
-            smem = smem_c;
+    // Widest window first: up to 128 projections for the bit mask of a seeding scan, 64 for explicit
+    // lists (the refine's grids), 32 for the 8-bit codes, 16 where a tile keeps a row set per trial
+    // (30,000 voxels with 1-64 candidates: 12.6 ms at 16, 14.5 at 32, 15.5 at 8).  Of each, the
+    // most trials per CTA (at most the tile) that keep GRC_SCAN_BLOCKS CTAs within the budget; a
+    // tile below two trials per warp goes on to the next window.
+    // A completeness call that a larger tile makes one round takes it.
+    if (MODE == kScanComp && !caller_tile && !explicit_voxels &&
+        n_trials <= (int64_t)GRC_SCAN_BLOCKS * num_sms * kScanSlots)
+        max_slots = kScanSlots;
+    const bool row_per_trial = rows_for(kScanSlotsBulk) == kScanSlotsBulk;
+    int win = 0, tile = 0, ctas = GRC_SCAN_BLOCKS;
+    for (; ctas >= 1 && !win; --ctas)
+        for (int cand : {128, 64, 32, 16, kScanWinMin}) {
+            if (cand > (MODE == kScanFull ? (row_per_trial ? 16 : 32) : explicit_voxels ? 64 : 128)) continue;
+            if (MODE == kScanComp && cand > 32 && (int64_t)cand * b.plane_words * 4 > l2_budget) continue;
+            if (MODE == kScanFull && cand > kScanWinMin && (int64_t)cand * g.plane > 2147483647LL) continue;
+            int t = max_slots;
+            while (t > 0 && ctas * (scan_smem_layout(MODE, g.nhkl, rows_for(t), t, cand, offs) + 1024) > kSmSmemBudget)
+                --t;
+            if (caller_tile ? t < max_slots : t < 2 * kWarps) continue;
+            win = cand;
+            tile = t;
             break;
         }
+    if (!win) {  // one CTA per SM, of what it can hold
+        win = kScanWinMin;
+        tile = caller_tile ? max_slots : 2 * kWarps;
+    } else {
+        ++ctas;
     }
-    if (refused) cudaGetLastError();  // a refused window query is not an error of this launch
+    int per_sm = 0;
+    size_t smem = scan_smem_layout(MODE, g.nhkl, rows_for(tile), tile, win, offs);
+    cudaError_t e = occupancy_for((const void *)window_kernel(win), smem, &per_sm);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) return cudaErrorInvalidConfiguration;
+    if (win && per_sm > ctas && ctas >= 1) per_sm = ctas;
+    const int64_t grid = (int64_t)per_sm * num_sms;
+    // rounds of equal size, so that the last is not a sliver
+    const int64_t rounds = (n_trials + grid * tile - 1) / (grid * tile);
+    int slots = (int)((n_trials + rounds * grid - 1) / (rounds * grid));
+    if (slots < 1) slots = 1;
+    const int rows_cap = rows_for(slots);
+    smem = scan_smem_layout(MODE, g.nhkl, rows_cap, slots, win, offs);
+    const ScanFn kern = window_kernel(win);
     e = allow_smem((const void *)kern, smem);
     if (e != cudaSuccess) return e;
     const int64_t per_round = grid * slots;

@@ -496,8 +496,9 @@ int grc_set_timing(grc_ctx *ctx, int enable);
  * Scoring kernel selection: 0 = by size (default: the projection-window warp scan, which keeps
  * the map windows L2-resident and runs one trial per warp at a time, once a call holds 1/16 of a
  * round of trials -- 1,776 on 148 SMs -- when each voxel carries at least 64 orientations, or
- * half a round otherwise; the CTA sweep for full-output calls of more than two rounds; the
- * per-trial kernel below that), 1 = always the per-trial kernel,
+ * half a round otherwise; the CTA sweep for full-output calls of more than two rounds on
+ * geometries of fewer than 5,000 (projection, reflection) pairs; the per-trial kernel below those
+ * sizes), 1 = always the per-trial kernel,
  * 2 = always the CTA sweep (the same windows with the trials of a CTA mixed in its batches),
  * 3 = always the warp scan.  Results are identical; only speed differs.  Batches (grc_batch_*)
  * read the same codes for their tile choice.
