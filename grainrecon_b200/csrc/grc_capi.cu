@@ -43,7 +43,7 @@ struct grc_ctx {
     grc::MapCodes mc{};
     int64_t mz = 0, my = 0, mrot = 0;
     std::vector<float> h_vals;
-    DevBuf fgeo, fne, ftrial, fcost0, fcost1, fimp, fhw, geo_dev, rot_cs, hkl, pos, U, res, tvoxel, rlist, in1, in2, in3, out, items, torient, counts, offsets, tmp, counter, p1, bad, nm, sp_keys, sp_ids, sp_keys2, sp_ids2, cell_cnt, cell_off, pr_raw, pr_keys, pr_keys2, pr_ids, pr_ids2, pcount, nmloop;
+    DevBuf fgeo, fub, fne, ftrial, fcost1, fimp, fhw, geo_dev, rot_cs, hkl, pos, U, res, tvoxel, rlist, in1, in2, in3, out, items, torient, counts, offsets, tmp, counter, p1, bad, nm, sp_keys, sp_ids, sp_keys2, sp_ids2, cell_cnt, cell_off, pr_raw, pr_keys, pr_keys2, pr_ids, pr_ids2, pcount, nmloop;
     grc::Geo *geo_pinned = nullptr;  // staging of the per-launch geometry copy
     grc::Geo geo_up{};               // the geometry geo_dev holds (valid when geo_up_ok)
     bool geo_up_ok = false;
@@ -615,7 +615,7 @@ int grc_ctx_destroy(grc_ctx *ctx) {
         cudaStreamSynchronize(ctx->stream);
         cudaFreeHost(ctx->geo_pinned);
         if (ctx->nm_active) cudaFreeHost(ctx->nm_active);
-        DevBuf *all[] = {&ctx->nm, &ctx->sp_keys, &ctx->sp_ids, &ctx->sp_keys2, &ctx->sp_ids2, &ctx->cell_cnt, &ctx->cell_off, &ctx->pr_raw, &ctx->pr_keys, &ctx->pr_keys2, &ctx->pr_ids, &ctx->pr_ids2, &ctx->pcount, &ctx->fgeo, &ctx->fne, &ctx->ftrial, &ctx->fcost0, &ctx->fcost1, &ctx->fimp, &ctx->fhw,
+        DevBuf *all[] = {&ctx->nm, &ctx->sp_keys, &ctx->sp_ids, &ctx->sp_keys2, &ctx->sp_ids2, &ctx->cell_cnt, &ctx->cell_off, &ctx->pr_raw, &ctx->pr_keys, &ctx->pr_keys2, &ctx->pr_ids, &ctx->pr_ids2, &ctx->pcount, &ctx->fgeo, &ctx->fub, &ctx->fne, &ctx->ftrial, &ctx->fcost1, &ctx->fimp, &ctx->fhw,
                          &ctx->tvoxel, &ctx->rlist, &ctx->geo_dev, &ctx->rot_cs, &ctx->hkl, &ctx->pos, &ctx->U, &ctx->res, &ctx->in1, &ctx->in2,
                          &ctx->in3, &ctx->out, &ctx->items, &ctx->torient, &ctx->counts, &ctx->offsets,
                          &ctx->tmp, &ctx->counter, &ctx->p1, &ctx->bad, &ctx->bits, &ctx->gkey,
@@ -2145,6 +2145,15 @@ grc::SpotList spots_of(const int32_t *g, const int32_t *w, const int32_t *h, con
     return sp;
 }
 
+// U*B of the spots' grains in the context's table.
+int grain_table(grc_ctx *ctx, const grc::FitFixed &fx, const double *d_grains, const grc::SpotList &sp,
+                const double **ub) {
+    TRY(ensure(ctx, ctx->fub, sizeof(double) * 9 * grc::kFitGrainTable));
+    CU(grc::fit_grain_ub(fx, d_grains, sp, (double *)ctx->fub.p, ctx->stream));
+    *ub = (const double *)ctx->fub.p;
+    return GRC_OK;
+}
+
 }  // namespace
 
 extern "C" int grc_fit_spot_count(grc_ctx *ctx, const double *geo10, const double *d_grains, int64_t n_grains,
@@ -2187,8 +2196,10 @@ extern "C" int grc_centroid_residual_adjoint(grc_ctx *ctx, int mode, const doubl
     grc::FitFixed fx;
     TRY(fit_prepare(ctx, geo10, &fx));
     if (n_spots == 0) return GRC_OK;
-    CU(grc::fit_residual_jacobian(fx, mode, d_grains, (const double *)ctx->fgeo.p,
-                                  spots_of(d_grain, d_iw, d_ih, d_uv, n_spots), d_res, d_jac, ctx->stream));
+    const grc::SpotList sp = spots_of(d_grain, d_iw, d_ih, d_uv, n_spots);
+    const double *ub = nullptr;
+    TRY(grain_table(ctx, fx, d_grains, sp, &ub));
+    CU(grc::fit_residual_jacobian(fx, mode, d_grains, ub, (const double *)ctx->fgeo.p, sp, d_res, d_jac, ctx->stream));
     CU(cudaStreamSynchronize(ctx->stream));
     return GRC_OK;
 }
@@ -2203,25 +2214,14 @@ extern "C" int grc_fit_grains_lm(grc_ctx *ctx, const double *geo10, double *d_gr
         return fail(ctx, GRC_EINVAL, "fit: bad arguments");
     grc::FitFixed fx;
     TRY(fit_prepare(ctx, geo10, &fx));
-    TRY(ensure(ctx, ctx->fne, sizeof(double) * 29 * n_grains));
-    TRY(ensure(ctx, ctx->ftrial, sizeof(double) * 6 * n_grains));
-    TRY(ensure(ctx, ctx->fcost0, sizeof(double) * 2 * n_grains));
-    TRY(ensure(ctx, ctx->fcost1, sizeof(double) * 2 * n_grains));
     TRY(ensure(ctx, ctx->fimp, sizeof(int)));
     const grc::SpotList sp = spots_of(d_grain, d_iw, d_ih, d_uv, n_spots);
     const double *g10 = (const double *)ctx->fgeo.p;
     int improved = 0;
     for (int it = 0; it < iters; ++it) {
         CU(cudaMemsetAsync(ctx->fimp.p, 0, sizeof(int), ctx->stream));
-        CU(grc::fit_grain_normal(fx, d_grains, g10, sp, d_offsets, n_grains, (double *)ctx->fne.p, ctx->stream));
-        CU(grc::fit_grain_cost(fx, d_grains, g10, sp, d_offsets, n_grains, (double *)ctx->fcost0.p, ctx->stream));
-        CU(grc::fit_grain_lm_propose(d_grains, (const double *)ctx->fne.p, d_lambda, n_grains,
-                                     (double *)ctx->ftrial.p, ctx->stream));
-        CU(grc::fit_grain_cost(fx, (const double *)ctx->ftrial.p, g10, sp, d_offsets, n_grains,
-                               (double *)ctx->fcost1.p, ctx->stream));
-        CU(grc::fit_grain_lm_accept(d_grains, (const double *)ctx->ftrial.p, (const double *)ctx->fcost0.p,
-                                    (const double *)ctx->fcost1.p, d_lambda, n_grains, (int *)ctx->fimp.p,
-                                    ctx->stream));
+        CU(grc::fit_grain_lm(fx, d_grains, g10, sp, d_offsets, n_grains, d_lambda, (int *)ctx->fimp.p, ctx->num_sms,
+                             ctx->stream));
         CU(cudaMemcpyAsync(&improved, ctx->fimp.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
         CU(cudaStreamSynchronize(ctx->stream));
         if (improved == 0) break;
@@ -2276,20 +2276,21 @@ extern "C" int grc_fit_geometry_lm(grc_ctx *ctx, double *d_starts, int n_starts,
     TRY(fit_prepare(ctx, nullptr, &fx));
     TRY(ensure(ctx, ctx->fne, sizeof(double) * 67 * n_starts));
     TRY(ensure(ctx, ctx->ftrial, sizeof(double) * 10 * n_starts));
-    TRY(ensure(ctx, ctx->fcost0, sizeof(double) * 2 * n_starts));
     TRY(ensure(ctx, ctx->fcost1, sizeof(double) * 2 * n_starts));
     TRY(ensure(ctx, ctx->fimp, sizeof(int)));
     const grc::SpotList sp = spots_of(d_grain, d_iw, d_ih, d_uv, n_spots);
+    const double *ub = nullptr;
+    TRY(grain_table(ctx, fx, d_grains, sp, &ub));
     int improved = 0;
     for (int it = 0; it < iters; ++it) {
         CU(cudaMemsetAsync(ctx->fimp.p, 0, sizeof(int), ctx->stream));
-        CU(grc::fit_geo_normal(fx, d_grains, d_starts, n_starts, sp, (double *)ctx->fne.p, ctx->num_sms, ctx->stream));
-        CU(grc::fit_geo_cost(fx, d_grains, d_starts, n_starts, sp, (double *)ctx->fcost0.p, ctx->num_sms, ctx->stream));
+        CU(grc::fit_geo_normal(fx, d_grains, ub, d_starts, n_starts, sp, (double *)ctx->fne.p, ctx->num_sms,
+                               ctx->stream));
         CU(grc::fit_geo_lm_propose(d_starts, (const double *)ctx->fne.p, d_lambda, n_starts, (double *)ctx->ftrial.p,
                                    ctx->stream));
-        CU(grc::fit_geo_cost(fx, d_grains, (const double *)ctx->ftrial.p, n_starts, sp, (double *)ctx->fcost1.p,
+        CU(grc::fit_geo_cost(fx, d_grains, ub, (const double *)ctx->ftrial.p, n_starts, sp, (double *)ctx->fcost1.p,
                              ctx->num_sms, ctx->stream));
-        CU(grc::fit_geo_lm_accept(d_starts, (const double *)ctx->ftrial.p, (const double *)ctx->fcost0.p,
+        CU(grc::fit_geo_lm_accept(d_starts, (const double *)ctx->ftrial.p, (const double *)ctx->fne.p, n_spots,
                                   (const double *)ctx->fcost1.p, d_lambda, n_starts, (int *)ctx->fimp.p, ctx->stream));
         CU(cudaMemcpyAsync(&improved, ctx->fimp.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
         CU(cudaStreamSynchronize(ctx->stream));
@@ -2308,8 +2309,10 @@ extern "C" int grc_fit_geometry_cost(grc_ctx *ctx, const double *d_points, int n
         return fail(ctx, GRC_EINVAL, "fit: bad arguments");
     grc::FitFixed fx;
     TRY(fit_prepare(ctx, nullptr, &fx));
-    CU(grc::fit_geo_cost(fx, d_grains, d_points, n_points, spots_of(d_grain, d_iw, d_ih, d_uv, n_spots), d_cost,
-                         ctx->num_sms, ctx->stream));
+    const grc::SpotList sp = spots_of(d_grain, d_iw, d_ih, d_uv, n_spots);
+    const double *ub = nullptr;
+    TRY(grain_table(ctx, fx, d_grains, sp, &ub));
+    CU(grc::fit_geo_cost(fx, d_grains, ub, d_points, n_points, sp, d_cost, ctx->num_sms, ctx->stream));
     CU(cudaStreamSynchronize(ctx->stream));
     return GRC_OK;
 }
@@ -2323,8 +2326,11 @@ extern "C" int grc_fit_geometry_rms(grc_ctx *ctx, const double *d_starts, int n_
         return fail(ctx, GRC_EINVAL, "fit: bad arguments");
     grc::FitFixed fx;
     TRY(fit_prepare(ctx, geo_truth10, &fx));
-    CU(grc::fit_geo_rms(fx, d_grains, d_starts, n_starts, (const double *)ctx->fgeo.p,
-                        spots_of(d_grain, d_iw, d_ih, d_uv, n_spots), d_acc, ctx->num_sms, ctx->stream));
+    const grc::SpotList sp = spots_of(d_grain, d_iw, d_ih, d_uv, n_spots);
+    const double *ub = nullptr;
+    TRY(grain_table(ctx, fx, d_grains, sp, &ub));
+    CU(grc::fit_geo_rms(fx, d_grains, ub, d_starts, n_starts, (const double *)ctx->fgeo.p, sp, d_acc, ctx->num_sms,
+                        ctx->stream));
     CU(cudaStreamSynchronize(ctx->stream));
     return GRC_OK;
 }
