@@ -41,6 +41,7 @@ struct grc_ctx {
     grc::Geo geo{};
     bool has_masks = false;
     grc::MapCodes mc{};
+    grc::Scratch map_ws[3];  // rank coding (2), distance transform
     int64_t mz = 0, my = 0, mrot = 0;
     std::vector<float> h_vals;
     DevBuf fgeo, fub, fne, ftrial, fcost1, fimp, fhw, geo_dev, rot_cs, hkl, pos, U, res, tvoxel, rlist, in1, in2, in3, out, items, torient, counts, offsets, tmp, counter, p1, bad, nm, sp_keys, sp_ids, sp_keys2, sp_ids2, cell_cnt, cell_off, pr_raw, pr_keys, pr_keys2, pr_ids, pr_ids2, pcount, nmloop;
@@ -231,27 +232,15 @@ int set_geometry(grc_ctx *ctx, const float *S, const float *B, const float *hkl,
 
 int upload_device_map(grc_ctx *ctx, const float *d_map, int64_t dz, int64_t dy, int64_t nrot) {
     const int64_t n = dz * dy * nrot;
-    grc::MapCodes mc{};
     int bad = 0;
-    cudaError_t e = grc::encode_map(d_map, n, ctx->stream, &mc, &bad);
+    cudaError_t e = grc::encode_map(d_map, n, ctx->stream, &ctx->mc, ctx->map_ws, &bad);
     if (e != cudaSuccess) return fail(ctx, GRC_ECUDA, "distance-map coding: %s", cudaGetErrorString(e));
     if (bad) return fail(ctx, GRC_EINVAL, "distance map holds NaN values");
-    std::vector<float> hv((size_t)mc.n_distinct);
-    if (mc.n_distinct > 0) {
-        e = cudaMemcpy(hv.data(), mc.vals, sizeof(float) * mc.n_distinct, cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) {
-            cudaFree(mc.codes);
-            cudaFree(mc.codes8);
-            cudaFree(mc.vals);
-            return fail(ctx, GRC_ECUDA, "value table copy: %s", cudaGetErrorString(e));
-        }
-    }
-    if (ctx->has_masks) {
-        cudaFree(ctx->mc.codes);
-        cudaFree(ctx->mc.codes8);
-        cudaFree(ctx->mc.vals);
-    }
-    ctx->mc = mc;
+    // from here the codes are the new map's: without its values there is no map
+    ctx->has_masks = false;
+    std::vector<float> hv((size_t)ctx->mc.n_distinct);
+    e = cudaMemcpy(hv.data(), ctx->mc.vals, sizeof(float) * hv.size(), cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) return fail(ctx, GRC_ECUDA, "value table copy: %s", cudaGetErrorString(e));
     ctx->bits_ok = false;  // packed again from the new codes when first needed
     ctx->map_key = 0;      // an upload that came without a key
     ctx->h_vals.swap(hv);
@@ -621,11 +610,8 @@ int grc_ctx_destroy(grc_ctx *ctx) {
                          &ctx->tmp, &ctx->counter, &ctx->p1, &ctx->bad, &ctx->bits, &ctx->gkey,
                          &ctx->sgrid, &ctx->sgrid32, &ctx->stv, &ctx->sto, &ctx->sbest, &ctx->nmloop};
         for (DevBuf *b : all) cudaFree(b->p);
-        if (ctx->has_masks) {
-            cudaFree(ctx->mc.codes);
-            cudaFree(ctx->mc.codes8);
-            cudaFree(ctx->mc.vals);
-        }
+        ctx->mc.release();
+        for (grc::Scratch &w : ctx->map_ws) w.release();
         cudaEventDestroy(ctx->ev0);
         cudaEventDestroy(ctx->ev1);
         cudaStreamDestroy(ctx->stream);
@@ -1179,7 +1165,7 @@ int upload_spot_device(grc_ctx *ctx, const uint8_t *d_mask, int64_t dz, int64_t 
     float *d_map = nullptr;
     cudaError_t e = cudaMalloc(&d_map, sizeof(float) * n);
     if (e != cudaSuccess) return fail(ctx, GRC_ECUDA, "cudaMalloc(distance map): %s", cudaGetErrorString(e));
-    e = grc::launch_edt(d_mask, dz, dy, nrot, d_map, ctx->stream);
+    e = grc::launch_edt(d_mask, dz, dy, nrot, d_map, &ctx->map_ws[2], ctx->stream);
     int r = e == cudaSuccess ? upload_device_map(ctx, d_map, dz, dy, nrot)
                              : fail(ctx, GRC_ECUDA, "bwdist: %s", cudaGetErrorString(e));
     cudaStreamSynchronize(ctx->stream);
@@ -1673,7 +1659,7 @@ int grc_edt(grc_ctx *ctx, const uint8_t *d_mask, int64_t dz, int64_t dy, int64_t
     Lock l(ctx);
     if (!d_mask || !d_map) return fail(ctx, GRC_EINVAL, "NULL device buffer");
     if (dz < 1 || dy < 1 || nrot < 1) return fail(ctx, GRC_EINVAL, "dimensions must be positive");
-    CU(grc::launch_edt(d_mask, dz, dy, nrot, d_map, ctx->stream));
+    CU(grc::launch_edt(d_mask, dz, dy, nrot, d_map, &ctx->map_ws[2], ctx->stream));
     return GRC_OK;
 }
 

@@ -179,21 +179,37 @@ cudaError_t launch_epi_compete(const TrialRes *res, const longlong4 *items, cons
 cudaError_t launch_apply_compete(const float *out8, const float *rows5, int64_t m, const int64_t *dims, float *comp,
                                  float *gid, float *dmed, float *ninter, float *visit, cudaStream_t s);
 
+// Device scratch of a context, kept between calls up to kKeep bytes; a larger request is served once
+// and given back by done().
+struct Scratch {
+    static constexpr size_t kKeep = size_t(64) << 20;
+    void *p = nullptr, *once = nullptr;
+    size_t cap = 0;
+    cudaError_t get(size_t bytes, cudaStream_t s, void **out);
+    void done(cudaStream_t s);
+    void release();
+};
+
 // Distance-map rank coding.
 struct MapCodes {
-    void *codes;
-    uint8_t *codes8;
-    float *vals;
-    int64_t n_distinct;
-    int code_bits;
+    void *codes = nullptr;
+    uint8_t *codes8 = nullptr;
+    float *vals = nullptr;
+    int64_t n_distinct = 0;
+    int code_bits = 0;
+    size_t cap_codes = 0, cap_codes8 = 0, cap_vals = 0;  // bytes allocated
+    void release();
 };
-// Encodes d_map (n floats) into codes; allocates codes/vals with cudaMalloc.
-cudaError_t encode_map(const float *d_map, int64_t n, cudaStream_t s, MapCodes *out, int *bad_nan);
+// Encodes d_map (n floats) into *resident, whose buffers are reused where they fit.  A map with NaN
+// values (*bad_nan) or a failed call leaves *resident valid; nothing of it is written before the map is
+// known to be good and every buffer allocated.  ws: two scratches.
+cudaError_t encode_map(const float *d_map, int64_t n, cudaStream_t s, MapCodes *resident, Scratch *ws, int *bad_nan);
 
 // Synthetic-data kernels.
 cudaError_t launch_simulate_work(const Geo &g, const ScoreBufs &b, const Work &w, int num_sms, uint8_t *mask,
                                  cudaStream_t s);
-cudaError_t launch_edt(const uint8_t *mask, int64_t nz, int64_t ny, int64_t nrot, float *map, cudaStream_t s);
+cudaError_t launch_edt(const uint8_t *mask, int64_t nz, int64_t ny, int64_t nrot, float *map, Scratch *ws,
+                       cudaStream_t s);
 
 // Spot pairing (grc_score.cu: pair_kernel; index built in grc_seed.cu).  Same layout as the
 // public grc_spot_pair.
