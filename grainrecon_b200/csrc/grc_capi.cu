@@ -44,7 +44,7 @@ struct grc_ctx {
     grc::Scratch map_ws[3];  // rank coding (2), distance transform
     int64_t mz = 0, my = 0, mrot = 0;
     std::vector<float> h_vals;
-    DevBuf fgeo, fub, fne, ftrial, fcost1, fimp, fhw, geo_dev, rot_cs, hkl, pos, U, res, tvoxel, rlist, in1, in2, in3, out, items, torient, counts, offsets, tmp, counter, p1, bad, nm, sp_keys, sp_ids, sp_keys2, sp_ids2, cell_cnt, cell_off, pr_raw, pr_keys, pr_keys2, pr_ids, pr_ids2, pcount, nmloop;
+    DevBuf fgeo, fub, fne, ftrial, fcost1, fimp, fhw, geo_dev, rot_cs, hkl, pos, U, res, tvoxel, rlist, in1, in2, in3, out, items, torient, counts, offsets, tmp, counter, p1, bad, nm, sp_keys, sp_ids, sp_keys2, sp_ids2, sp_yz, cell_cnt, cell_off, pr_rec, pr_units, pcount, nmloop;
     grc::Geo *geo_pinned = nullptr;  // staging of the per-launch geometry copy
     grc::Geo geo_up{};               // the geometry geo_dev holds (valid when geo_up_ok)
     bool geo_up_ok = false;
@@ -604,7 +604,7 @@ int grc_ctx_destroy(grc_ctx *ctx) {
         cudaStreamSynchronize(ctx->stream);
         cudaFreeHost(ctx->geo_pinned);
         if (ctx->nm_active) cudaFreeHost(ctx->nm_active);
-        DevBuf *all[] = {&ctx->nm, &ctx->sp_keys, &ctx->sp_ids, &ctx->sp_keys2, &ctx->sp_ids2, &ctx->cell_cnt, &ctx->cell_off, &ctx->pr_raw, &ctx->pr_keys, &ctx->pr_keys2, &ctx->pr_ids, &ctx->pr_ids2, &ctx->pcount, &ctx->fgeo, &ctx->fub, &ctx->fne, &ctx->ftrial, &ctx->fcost1, &ctx->fimp, &ctx->fhw,
+        DevBuf *all[] = {&ctx->nm, &ctx->sp_keys, &ctx->sp_ids, &ctx->sp_keys2, &ctx->sp_ids2, &ctx->sp_yz, &ctx->cell_cnt, &ctx->cell_off, &ctx->pr_rec, &ctx->pr_units, &ctx->pcount, &ctx->fgeo, &ctx->fub, &ctx->fne, &ctx->ftrial, &ctx->fcost1, &ctx->fimp, &ctx->fhw,
                          &ctx->tvoxel, &ctx->rlist, &ctx->geo_dev, &ctx->rot_cs, &ctx->hkl, &ctx->pos, &ctx->U, &ctx->res, &ctx->in1, &ctx->in2,
                          &ctx->in3, &ctx->out, &ctx->items, &ctx->torient, &ctx->counts, &ctx->offsets,
                          &ctx->tmp, &ctx->counter, &ctx->p1, &ctx->bad, &ctx->bits, &ctx->gkey,
@@ -1494,7 +1494,7 @@ int grc_pair_spots(grc_ctx *ctx, const double *d_pos, const double *d_q, int64_t
     if (n > (int64_t)INT32_MAX || n_spots > (int64_t)INT32_MAX)
         return fail(ctx, GRC_ECAPACITY, "pair: more than 2^31-1 trials or spots");
     const grc::Geo &g = ctx->geo;
-    constexpr int kCell = 16;
+    constexpr int kCell = grc::kSpotCell;
     const int ncy = (g.detysize + kCell - 1) / kCell, ncz = (g.detzsize + kCell - 1) / kCell;
     const int64_t ncell = (int64_t)g.nrot * ncy * ncz;
     cudaStream_t s = ctx->stream;
@@ -1508,22 +1508,26 @@ int grc_pair_spots(grc_ctx *ctx, const double *d_pos, const double *d_q, int64_t
         if (off[i + 1] < off[i]) return fail(ctx, GRC_EINVAL, "pair: projection offsets decrease at %d", i);
     TRY(ensure(ctx, ctx->U, sizeof(double) * 9 * n));
     TRY(ensure(ctx, ctx->pos, sizeof(double) * 3 * n));
-    TRY(ensure(ctx, ctx->cell_cnt, sizeof(int64_t) * (ncell + 1)));
-    TRY(ensure(ctx, ctx->cell_off, sizeof(int64_t) * (ncell + 1)));
+    TRY(ensure(ctx, ctx->cell_cnt, sizeof(int32_t) * (ncell + 1)));
+    TRY(ensure(ctx, ctx->cell_off, sizeof(int32_t) * (ncell + 1)));
+    TRY(ensure(ctx, ctx->sp_yz, sizeof(double) * 2 * (n_spots + 1)));
     TRY(ensure(ctx, ctx->sp_keys, sizeof(int32_t) * (n_spots + 1)));
     TRY(ensure(ctx, ctx->sp_ids, sizeof(int32_t) * (n_spots + 1)));
     TRY(ensure(ctx, ctx->sp_keys2, sizeof(int32_t) * (n_spots + 1)));
     TRY(ensure(ctx, ctx->sp_ids2, sizeof(int32_t) * (n_spots + 1)));
     TRY(ensure(ctx, ctx->pcount, sizeof(unsigned long long)));
-    TRY(ensure(ctx, ctx->pr_raw, sizeof(grc::PairRec) * (max_pairs > 0 ? max_pairs : 1)));
+    // no more pairs than (projection, reflection) pairs of all trials
+    const int64_t room = std::min<int64_t>(max_pairs, n * g.nrot * g.nhkl), units = grc::pair_units(g, n);
+    TRY(ensure(ctx, ctx->pr_rec, sizeof(uint4) * (room > 0 ? room : 1)));
+    TRY(ensure(ctx, ctx->pr_units, sizeof(int64_t) * 3 * units));
     CU(grc::launch_quat_to_u_d(d_q, n, (double *)ctx->U.p, s));
     CU(cudaMemcpyAsync(ctx->pos.p, d_pos, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice, s));
-    CU(cudaMemsetAsync(ctx->cell_cnt.p, 0, sizeof(int64_t) * (ncell + 1), s));
+    CU(cudaMemsetAsync(ctx->cell_cnt.p, 0, sizeof(int32_t) * (ncell + 1), s));
     int end_bit = 1;
     while (end_bit < 31 && ((int64_t)1 << end_bit) < ncell) ++end_bit;
     if (n_spots > 0) {
-        CU(grc::launch_spot_keys(d_spots, d_proj_offsets, g.nrot, ncy, ncz, kCell, (int32_t *)ctx->sp_keys.p,
-                                 (int32_t *)ctx->sp_ids.p, (int64_t *)ctx->cell_cnt.p, s));
+        CU(grc::launch_spot_keys(d_spots, d_proj_offsets, g.nrot, ncy, ncz, (int32_t *)ctx->sp_keys.p,
+                                 (int32_t *)ctx->sp_ids.p, (int32_t *)ctx->cell_cnt.p, s));
         size_t tb = 0;
         CU(cub::DeviceRadixSort::SortPairs(nullptr, tb, (const int32_t *)ctx->sp_keys.p, (int32_t *)ctx->sp_keys2.p,
                                            (const int32_t *)ctx->sp_ids.p, (int32_t *)ctx->sp_ids2.p, n_spots, 0,
@@ -1532,52 +1536,42 @@ int grc_pair_spots(grc_ctx *ctx, const double *d_pos, const double *d_q, int64_t
         CU(cub::DeviceRadixSort::SortPairs(ctx->tmp.p, tb, (const int32_t *)ctx->sp_keys.p, (int32_t *)ctx->sp_keys2.p,
                                            (const int32_t *)ctx->sp_ids.p, (int32_t *)ctx->sp_ids2.p, n_spots, 0,
                                            end_bit, s));
+        CU(grc::launch_spot_gather(d_spots, (const int32_t *)ctx->sp_ids2.p, n_spots, (double *)ctx->sp_yz.p, s));
     }
     {
         size_t tb = 0;
-        CU(cub::DeviceScan::ExclusiveSum(nullptr, tb, (int64_t *)ctx->cell_cnt.p, (int64_t *)ctx->cell_off.p,
+        CU(cub::DeviceScan::ExclusiveSum(nullptr, tb, (int32_t *)ctx->cell_cnt.p, (int32_t *)ctx->cell_off.p,
                                          ncell + 1, s));
         TRY(ensure(ctx, ctx->tmp, tb));
-        CU(cub::DeviceScan::ExclusiveSum(ctx->tmp.p, tb, (int64_t *)ctx->cell_cnt.p, (int64_t *)ctx->cell_off.p,
+        CU(cub::DeviceScan::ExclusiveSum(ctx->tmp.p, tb, (int32_t *)ctx->cell_cnt.p, (int32_t *)ctx->cell_off.p,
                                          ncell + 1, s));
     }
-    grc::SpotIndex si{d_spots, (const int64_t *)ctx->cell_off.p, (const int32_t *)ctx->sp_ids2.p, ncy, ncz, kCell};
+    grc::SpotIndex si{d_spots, (const int32_t *)ctx->cell_off.p, (const int32_t *)ctx->sp_ids2.p,
+                      (const double *)ctx->sp_yz.p, ncy, ncz};
     CU(cudaMemsetAsync(ctx->pcount.p, 0, sizeof(unsigned long long), s));
     TRY(stage_geo(ctx));
-    CU(grc::launch_pair(g, bufs(ctx), n, si, (grc::PairRec *)ctx->pr_raw.p, max_pairs,
-                        (unsigned long long *)ctx->pcount.p, ctx->num_sms, s));
+    grc::PairUnits u{};
+    u.count = (int64_t *)ctx->pr_units.p;
+    u.seg = u.count + units;
+    u.base = u.seg + units;
+    u.rec = (uint4 *)ctx->pr_rec.p;
+    u.cap = room;
+    u.total = (unsigned long long *)ctx->pcount.p;
+    CU(grc::launch_pair_find(g, bufs(ctx), n, si, u, ctx->num_sms, s));
+    {
+        size_t tb = 0;
+        CU(cub::DeviceScan::ExclusiveSum(nullptr, tb, u.count, u.base, units, s));
+        TRY(ensure(ctx, ctx->tmp, tb));
+        CU(cub::DeviceScan::ExclusiveSum(ctx->tmp.p, tb, u.count, u.base, units, s));
+    }
+    if (max_pairs > 0) CU(grc::launch_pair_write(g, bufs(ctx), n, si, u, (grc::PairRec *)d_pairs, ctx->num_sms, s));
     unsigned long long cnt = 0;
     CU(cudaMemcpyAsync(&cnt, ctx->pcount.p, sizeof(cnt), cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
     *n_pairs = (int64_t)cnt;
     if ((int64_t)cnt > max_pairs) return fail(ctx, GRC_ECAPACITY, "pair: %llu pairs exceed max_pairs", cnt);
-    if (cnt > 0) {
-        // atomics leave the pairs in arbitrary order: sort by (trial, projection, reflection)
-        const int64_t m = (int64_t)cnt;
-        TRY(ensure(ctx, ctx->pr_keys, sizeof(int64_t) * m));
-        TRY(ensure(ctx, ctx->pr_keys2, sizeof(int64_t) * m));
-        TRY(ensure(ctx, ctx->pr_ids, sizeof(int32_t) * m));
-        TRY(ensure(ctx, ctx->pr_ids2, sizeof(int32_t) * m));
-        CU(grc::launch_pair_keys((const grc::PairRec *)ctx->pr_raw.p, m, g.nrot, g.nhkl, (int64_t *)ctx->pr_keys.p,
-                                 (int32_t *)ctx->pr_ids.p, s));
-        // keys (trial * nrot + iw) * nhkl + ih are below n * nrot * nhkl: sort only those bits
-        const uint64_t key_end = (uint64_t)n * (uint64_t)g.nrot * (uint64_t)g.nhkl;
-        int key_bits = 1;
-        while (key_bits < 63 && (uint64_t(1) << key_bits) < key_end) ++key_bits;
-        size_t tb = 0;
-        CU(cub::DeviceRadixSort::SortPairs(nullptr, tb, (const int64_t *)ctx->pr_keys.p, (int64_t *)ctx->pr_keys2.p,
-                                           (const int32_t *)ctx->pr_ids.p, (int32_t *)ctx->pr_ids2.p, m, 0, key_bits,
-                                           s));
-        TRY(ensure(ctx, ctx->tmp, tb));
-        CU(cub::DeviceRadixSort::SortPairs(ctx->tmp.p, tb, (const int64_t *)ctx->pr_keys.p, (int64_t *)ctx->pr_keys2.p,
-                                           (const int32_t *)ctx->pr_ids.p, (int32_t *)ctx->pr_ids2.p, m, 0, key_bits,
-                                           s));
-        CU(grc::launch_pair_gather((const grc::PairRec *)ctx->pr_raw.p, (const int32_t *)ctx->pr_ids2.p, m,
-                                   (grc::PairRec *)d_pairs, s));
-        CU(cudaStreamSynchronize(s));
-    }
     ctx->stats.trials = n;
-    ctx->stats.kernel_launches = 6 + (cnt > 0 ? 3 : 0);
+    ctx->stats.kernel_launches = 8;
     return GRC_OK;
 }
 

@@ -217,20 +217,32 @@ struct PairRec {
     int32_t trial, iw, ih, spot;
     double dety, detz, exp_y, exp_z, area, energy_kev, dis;
 };
+constexpr int kSpotCell = 16;  // side of the spot index's cells [pixel]
 struct SpotIndex {
     const double *yza;        // 3 per spot: centroid dety, detz [pixel], area [pixel^2]
-    const int64_t *cell_off;  // [nrot * ncy * ncz + 1]
+    const int32_t *cell_off;  // [nrot * ncy * ncz + 1]
     const int32_t *cell_ids;  // spot ids in (projection, cell, list) order
-    int ncy, ncz, cell_px;
+    const double *yz;         // their centroids, in that order
+    int ncy, ncz;
 };
-cudaError_t launch_pair(const Geo &g, const ScoreBufs &b, int64_t n, const SpotIndex &si, PairRec *out, int64_t cap,
-                        unsigned long long *count, int num_sms, cudaStream_t s);
+// Units of a pairing call (pair_units of them): how many pairs each found, where its compact records lie
+// (a segment of rec, cap records in all) and where its result begins; `total` counts all pairs.
+struct PairUnits {
+    int64_t *count, *seg, *base;
+    uint4 *rec;
+    int64_t cap;
+    unsigned long long *total;
+};
+int64_t pair_units(const Geo &g, int64_t n);
+cudaError_t launch_pair_find(const Geo &g, const ScoreBufs &b, int64_t n, const SpotIndex &si, const PairUnits &u,
+                             int num_sms, cudaStream_t s);
+cudaError_t launch_pair_write(const Geo &g, const ScoreBufs &b, int64_t n, const SpotIndex &si, const PairUnits &u,
+                              PairRec *out, int num_sms, cudaStream_t s);
 // Cell index of a spot list: per spot its cell key ((iw * ncy + cy) * ncz + cz), then counts.
-cudaError_t launch_spot_keys(const double *yza, const int64_t *proj_off, int nrot, int ncy, int ncz, int cell_px,
-                             int32_t *keys, int32_t *ids, int64_t *cell_counts, cudaStream_t s);
-cudaError_t launch_pair_keys(const PairRec *p, int64_t n, int nrot, int nhkl, int64_t *keys, int32_t *ids,
-                             cudaStream_t s);
-cudaError_t launch_pair_gather(const PairRec *in, const int32_t *order, int64_t n, PairRec *out, cudaStream_t s);
+cudaError_t launch_spot_keys(const double *yza, const int64_t *proj_off, int nrot, int ncy, int ncz, int32_t *keys,
+                             int32_t *ids, int32_t *cell_counts, cudaStream_t s);
+// yz[2 q], yz[2 q + 1]: centroid of spot ids[q].
+cudaError_t launch_spot_gather(const double *yza, const int32_t *ids, int64_t n, double *yz, cudaStream_t s);
 
 // FP64 trial lists (grc_seed.cu): U from double quaternions, work items from (voxel, orientation)
 // index pairs (bad |= 1 for an index out of range; that item is left empty).
