@@ -112,6 +112,17 @@ __host__ __device__ inline size_t scan_smem_layout(int mode, int nhkl, int rows_
     return (o + 15) & ~size_t(15);
 }
 
+// Two FP32 multiply-adds in one instruction, each rounded as a scalar fma.
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
 __device__ __forceinline__ void cp_async4(uint32_t *dst, const uint32_t *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
                  : "memory");
@@ -198,7 +209,10 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
             o[0] = make_float4((float)d.kx, r.ky, r.kz, r.L2);
             o[WIN] = make_float4(r.cN, r.ay, r.az, r.num);
             o[2 * WIN] = make_float4(r.u0, r.v0, r.c, r.s);
-            o[3 * WIN] = make_float4(r.wx, r.wy, r.wz, 0.f);
+            float *kw = (float *)(sm.rows + (vl * kRowParts + 3) * WIN) + wl;
+            kw[0] = r.wx;
+            kw[WIN] = r.wy;
+            kw[2 * WIN] = r.wz;
         }
         if (tid == 0) s_next = 0;
         __syncthreads();
@@ -265,7 +279,8 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
                     const float4 gv = gw_of(sf, sm.hk[ih]);
                     const float4 wv = window_f(g, gv);
                     tab[2 * ih] = gv;
-                    tab[2 * ih + 1] = make_float4(wv.z, wv.w, 0.5f * (wv.x + wv.y), 0.5f * (wv.y - wv.x));
+                    tab[2 * ih + 1] = make_float4(wv.z, wv.w, 0.5f * (wv.x + wv.y),
+                                                  wv.y > wv.x ? 0.25f * (wv.y - wv.x) * (wv.y - wv.x) : -1.0f);
                 }
             }
             __syncwarp();
@@ -359,30 +374,39 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
                 while (k < nw) {
                     if (!tested) {
                         tested = true;
-                        float gx[HPL], gy[HPL], gz[HPL], mid[HPL], half[HPL];
+                        uint64_t gx[HPL], gy[HPL], gz[HPL], mid[HPL], nh2[HPL];
 #pragma unroll
                         for (int j = 0; j < HPL; ++j) {
                             const int ih = lane + 32 * j;
                             const bool real = ih < g.nhkl;
                             const float4 gv = tab[real ? 2 * ih : 0];
                             const float4 wv = tab[real ? 2 * ih + 1 : 1];
-                            gx[j] = gv.x;
-                            gy[j] = gv.y;
-                            gz[j] = gv.z;
-                            mid[j] = wv.z;
-                            half[j] = real ? wv.w : -1.0f;
+                            gx[j] = pack2(gv.x, gv.x);
+                            gy[j] = pack2(gv.y, gv.y);
+                            gz[j] = pack2(gv.z, gv.z);
+                            mid[j] = pack2(wv.z, wv.z);
+                            const float nh = real ? -wv.w : 1.0f;
+                            nh2[j] = pack2(nh, nh);
                             rem[j] = 0;
                         }
-                        const float4 *kw = vr + 3 * WIN + k;
-#pragma unroll 8
-                        for (int p = kSpan - 1; p >= 0; --p) {
-                            const float4 q = kw[p];
+                        const float *kw = (const float *)(vr + 3 * WIN) + k;
+#pragma unroll 4
+                        for (int p = kSpan - 4; p >= 0; p -= 4) {
+                            const ulonglong2 qx = *(const ulonglong2 *)(kw + p);
+                            const ulonglong2 qy = *(const ulonglong2 *)(kw + WIN + p);
+                            const ulonglong2 qz = *(const ulonglong2 *)(kw + 2 * WIN + p);
 #pragma unroll
                             for (int j = 0; j < HPL; ++j) {
-                                // |t - middle| - half is negative inside the window, t = -(k_w . Gw):
-                                // its sign bit joins the mask from below
-                                const float d = fmaf(q.x, gx[j], fmaf(q.y, gy[j], fmaf(q.z, gz[j], mid[j])));
-                                rem[j] = __funnelshift_l(__float_as_uint(fabsf(d) - half[j]), rem[j], 1);
+                                // (t - middle)^2 - half^2 is negative inside the window, t = -(k_w . Gw):
+                                // the sign bits of two projections at a time join the mask from below
+                                uint64_t d = fma2(qx.y, gx[j], fma2(qy.y, gy[j], fma2(qz.y, gz[j], mid[j])));
+                                d = fma2(d, d, nh2[j]);
+                                rem[j] = __funnelshift_l((uint32_t)(d >> 32), rem[j], 1);
+                                rem[j] = __funnelshift_l((uint32_t)d, rem[j], 1);
+                                d = fma2(qx.x, gx[j], fma2(qy.x, gy[j], fma2(qz.x, gz[j], mid[j])));
+                                d = fma2(d, d, nh2[j]);
+                                rem[j] = __funnelshift_l((uint32_t)(d >> 32), rem[j], 1);
+                                rem[j] = __funnelshift_l((uint32_t)d, rem[j], 1);
                             }
                         }
                         const uint32_t live = nw - k < 32 ? (1u << (nw - k)) - 1u : kAll;
