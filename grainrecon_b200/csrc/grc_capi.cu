@@ -137,14 +137,11 @@ void apply_options(grc_ctx *ctx) {
     g.dety0 = std::isnan(ctx->opt_dety0) ? g.detysize / 2.0 + 0.5 : ctx->opt_dety0;
     g.detz0 = std::isnan(ctx->opt_detz0) ? g.detzsize / 2.0 + 0.5 : ctx->opt_detz0;
     for (int i = 0; i < 9; ++i) g.Rf[i] = (float)g.R[i];
-    g.Ruf[0] = (float)(g.R[4] / g.pxy);
-    g.Ruf[1] = (float)(g.R[7] / g.pxy);
-    g.Rvf[0] = (float)(g.R[5] / g.pxz);
-    g.Rvf[1] = (float)(g.R[8] / g.pxz);
+    g.Ryf = make_float2((float)(g.R[4] / g.pxy), (float)(g.R[5] / g.pxz));
+    g.Rzf = make_float2((float)(g.R[7] / g.pxy), (float)(g.R[8] / g.pxz));
     g.rpxy = 1.0 / g.pxy;
     g.rpxz = 1.0 / g.pxz;
-    g.Raf[0] = (float)(g.R[1] / (g.R[0] * g.pxy));
-    g.Raf[1] = (float)(g.R[2] / (g.R[0] * g.pxz));
+    g.Raf = make_float2((float)(g.R[1] / (g.R[0] * g.pxy)), (float)(g.R[2] / (g.R[0] * g.pxz)));
     g.beam_stop = g.bsy0 <= g.bsy1 && g.bsy1 >= 1.0 && g.bsy0 <= g.detysize && g.bsz0 <= g.bsz1 && g.bsz1 >= 1.0 &&
                   g.bsz0 <= g.detzsize;
     g.dety0f = (float)g.dety0;

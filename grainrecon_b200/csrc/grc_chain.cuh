@@ -209,10 +209,38 @@ __device__ __forceinline__ float rcp_approx(float x) {
     return r;
 }
 
+// Two FP32 operations in one instruction, each rounded as the scalar one.
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ uint64_t pack2(float2 v) { return pack2(v.x, v.y); }
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
 // In-plane map offset of an FP32 landing (u, v): (dety-1)*detzsize + (detz-1), -1 for a certain
 // rejection, or -2 within the ambiguity band of a pixel edge or when `certain` is false.  Selects
 // instead of branches: the lanes of a batch part at every test.
-__device__ __forceinline__ int pixel_of(const Geo &g, float u, float v, bool certain) {
+__device__ __forceinline__ int pixel_of(const Geo &g, uint64_t uv, bool certain) {
     // nearest integer by the 1.5*2^23 addition: for |u| < 2^22 the sum's low mantissa bits hold the
     // rounded value, read back as an integer without a conversion instruction.  Within the
     // ambiguity band of a half-pixel the item goes to the exact path, so the tie rule of the
@@ -220,12 +248,12 @@ __device__ __forceinline__ int pixel_of(const Geo &g, float u, float v, bool cer
     // and more leaves an integer outside 1..10^6 (detectors have at most 10^6 pixels per side), a
     // certain rejection.
     constexpr float kRound = 12582912.0f;
-    const float tu = __fadd_rn(u, kRound), tv = __fadd_rn(v, kRound);
-    const float ru = __fsub_rn(tu, kRound), rv = __fsub_rn(tv, kRound);
-    certain = certain & (fabsf(u - ru) <= 0.5f - kAmbigPx) & (fabsf(v - rv) <= 0.5f - kAmbigPx);
-    const uint32_t iu = (uint32_t)(__float_as_int(tu) - 0x4B400001), iv = (uint32_t)(__float_as_int(tv) - 0x4B400001);
+    const uint64_t t2 = add2(uv, pack2(kRound, kRound)), r2 = add2(t2, pack2(-kRound, -kRound));
+    const float2 t = unpack2(t2), r = unpack2(r2), d = unpack2(fma2(r2, pack2(-1.0f, -1.0f), uv));
+    certain = certain & (fabsf(d.x) <= 0.5f - kAmbigPx) & (fabsf(d.y) <= 0.5f - kAmbigPx);
+    const uint32_t iu = (uint32_t)(__float_as_int(t.x) - 0x4B400001), iv = (uint32_t)(__float_as_int(t.y) - 0x4B400001);
     bool in = (iu < (uint32_t)g.detysize) & (iv < (uint32_t)g.detzsize);  // 0-based pixel
-    if (g.beam_stop) in = in & !((ru >= g.bsy0f) & (ru <= g.bsy1f) & (rv >= g.bsz0f) & (rv <= g.bsz1f));
+    if (g.beam_stop) in = in & !((r.x >= g.bsy0f) & (r.x <= g.bsy1f) & (r.y >= g.bsz0f) & (r.y <= g.bsz1f));
     const int ip = (int)(iu * (uint32_t)g.detzsize + iv);  // < 2^31 pixels per plane
     return certain ? (in ? ip : -1) : -2;
 }
@@ -256,8 +284,8 @@ __device__ __forceinline__ int landing_fp32(const Geo &g, const RowF &r, const f
     const float Ky = r.ay + diff * gy, Kz = r.az + diff * gz;  // K_x = ax lives in cN, cY, cZ
     const float nK = r.cN + g.Rf[3] * Ky + g.Rf[6] * Kz;
     const float f = __fdividef(r.num, nK);
-    const float u = r.u0 - f * (r.cY + g.Ruf[0] * Ky + g.Ruf[1] * Kz);
-    const float v = r.v0 - f * (r.cZ + g.Rvf[0] * Ky + g.Rvf[1] * Kz);
+    const float u = r.u0 - f * (r.cY + g.Ryf.x * Ky + g.Rzf.x * Kz);
+    const float v = r.v0 - f * (r.cZ + g.Ryf.y * Ky + g.Rzf.y * Kz);
     if (!(fabsf(u) < 2e6f && fabsf(v) < 2e6f)) {  // detectors have at most 10^6 pixels per side
         // far off the detector (or NaN): certain rejection only for finite values
         return (isfinite(u) && isfinite(v)) ? -1 : -2;
@@ -276,29 +304,30 @@ __device__ __forceinline__ int landing_fp32(const Geo &g, const RowF &r, const f
     return (int)((uint32_t)(iu - 1) * (uint32_t)g.detzsize + (uint32_t)(iv - 1));  // < 2^31 pixels per plane
 }
 
-// The same landing from a row of 12 numbers, {kx, ky, kz, L2}, {cN, ay, az, num}, {u0, v0, c, s}: cY
+// The same landing from a row of 12 numbers, {kx, L2, ky, kz}, {cN, num, ay, az}, {u0, v0, c, s}: cY
 // and cZ are multiples of cN, and k_in . (Omega Gw) is formed with the rotated G, so a lane reads
-// three 16-byte words of its projection instead of four.  A radicand below zero by rounding (x or
-// cphx beyond 1) gives NaN, so the exact path decides.
+// three 16-byte words of its projection instead of four, and y and z (u and v) go through together.
+// A radicand below zero by rounding (x or cphx beyond 1) gives NaN, so the exact path decides.
 __device__ __forceinline__ int landing_row3(const Geo &g, const float4 k, const float4 a, const float4 o,
                                             const float4 gw, float lo_in, float hi_in) {
     const float Gtx = o.z * gw.x - o.w * gw.y, Gty = o.w * gw.x + o.z * gw.y, Gtz = gw.z;
-    const float dot = k.x * Gtx + k.y * Gty + k.z * Gtz;
+    const float dot = k.x * Gtx + k.z * Gty + k.w * Gtz;
     const bool inside = (-dot > lo_in) & (-dot < hi_in);
     const float x = dot * gw.w, x2 = x * x;
     const float q = 1.0f - x2, c2 = 1.0f - 2.0f * x2;
     const float s2 = (-2.0f * x) * (q * rsq_approx(q));
     const float rk = rsq_approx(Gty * Gty + Gtz * Gtz);
-    const float gy = Gty * rk, gz = Gtz * rk;
-    const float cphx = gy * k.y + gz * k.z;
+    const uint64_t gt = mul2(pack2(Gty, Gtz), pack2(rk, rk));
+    const float2 gyz = unpack2(gt);
+    const float cphx = gyz.x * k.z + gyz.y * k.w;
     const float p = 1.0f - cphx * cphx;
     const float sphy = (p * rsq_approx(p)) * c2 - cphx * s2;
-    const float diff = (k.w * s2) * rcp_approx(sphy);
-    const float Ky = a.y + diff * gy, Kz = a.z + diff * gz;
-    const float f = a.w * rcp_approx(a.x + g.Rf[3] * Ky + g.Rf[6] * Kz);
-    const float u = o.x - f * (g.Raf[0] * a.x + (g.Ruf[0] * Ky + g.Ruf[1] * Kz));
-    const float v = o.y - f * (g.Raf[1] * a.x + (g.Rvf[0] * Ky + g.Rvf[1] * Kz));
-    return pixel_of(g, u, v, inside);
+    const float diff = (k.y * s2) * rcp_approx(sphy);
+    const float2 K = unpack2(fma2(pack2(diff, diff), gt, pack2(a.z, a.w)));
+    const float f = -a.y * rcp_approx(a.x + g.Rf[3] * K.x + g.Rf[6] * K.y);
+    const uint64_t ray = fma2(pack2(g.Raf), pack2(a.x, a.x),
+                              fma2(pack2(g.Ryf), pack2(K.x, K.x), mul2(pack2(g.Rzf), pack2(K.y, K.y))));
+    return pixel_of(g, fma2(pack2(f, f), ray, pack2(o.x, o.y)), inside);
 }
 
 // Gw (FP32) of one reflection from the slot's S*U*B and h; .w = 1/|Gw|.

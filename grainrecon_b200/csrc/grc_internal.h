@@ -26,8 +26,9 @@ struct Geo {
     double S[9], B[9], R[9]; // row-major
     // FP32 copies for the fast landing chain
     float Rf[9];
-    float Ruf[2], Rvf[2];    // R[4]/pxy, R[7]/pxy and R[5]/pxz, R[8]/pxz (ray K -> pixel u, v)
-    float Raf[2];            // R[1]/(R[0] pxy) and R[2]/(R[0] pxz) (the same for R[0] K_x)
+    // ray K -> pixel (u, v): K_y times Ryf = {R[4]/pxy, R[5]/pxz}, K_z times Rzf = {R[7]/pxy, R[8]/pxz}
+    // and R[0] K_x times Raf = {R[1]/(R[0] pxy), R[2]/(R[0] pxz)}
+    float2 Ryf, Rzf, Raf;
     float dety0f, detz0f, rpxyf, rpxzf;
     float bsy0f, bsy1f, bsz0f, bsz1f;
     int beam_stop;           // 0 when the beam stop covers no pixel of the detector

@@ -60,8 +60,8 @@ __device__ __forceinline__ int64_t scan_orient_of(const Work &w, int64_t t, int6
 }
 
 // Omega row of one (voxel, projection) as four float4 planes of WIN projections each, so that lanes
-// on consecutive projections read consecutive 16-byte words: {kx, ky, kz, L2}, {cN, ay, az, num},
-// {u0, v0, c, s} for the landing and {wx, wy, wz, -} = k_w for the window test.
+// on consecutive projections read consecutive 16-byte words: {kx, L2, ky, kz}, {cN, num, ay, az},
+// {u0, v0, c, s} for the landing, and k_w for the window test as planes of WIN floats wx, wy, wz.
 constexpr int kRowParts = 4;
 // Landings of a (trial, window) awaiting their batch: fewer than 64 left over plus one run of up to
 // 32 projections per lane, one mark bit each, in rings.
@@ -85,7 +85,7 @@ struct ScanSmem {
 constexpr int kExactCap = 128;                              // ambiguous items awaiting the FP64 path
 constexpr int kOffRuns = kMarkRing * 4;                     // [kRunRing]
 constexpr int kOffExact = kOffRuns + kRunRing * 4;          // [kExactCap]
-constexpr int kOffTable = kOffExact + kExactCap * 4;        // [nhkl] {Gw x, y, z, 1/|G|}, {certain lo, hi, middle, half}
+constexpr int kOffTable = kOffExact + kExactCap * 4;        // [nhkl] {Gw x, y, z, 1/|G|}, [nhkl] certain {lo, hi}, [nhkl] {middle, half^2}
 // ... and in full mode after it [kStages * 32] map words of the batches in flight
 __host__ __device__ inline size_t warp_block_bytes(int mode, int nhkl) {
     return kOffTable + sizeof(float4) * 2 * nhkl + (mode == kScanFull ? sizeof(uint32_t) * kStages * 32 : 0);
@@ -112,17 +112,6 @@ __host__ __device__ inline size_t scan_smem_layout(int mode, int nhkl, int rows_
     return (o + 15) & ~size_t(15);
 }
 
-// Two FP32 multiply-adds in one instruction, each rounded as a scalar fma.
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
-    uint64_t d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-    return d;
-}
 __device__ __forceinline__ void cp_async4(uint32_t *dst, const uint32_t *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
                  : "memory");
@@ -164,7 +153,8 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
     unsigned char *wb = sm.warps + warp * warp_block_bytes(MODE, g.nhkl);
     uint32_t *marks = (uint32_t *)wb, *runs = (uint32_t *)(wb + kOffRuns), *fq = (uint32_t *)(wb + kOffExact);
     float4 *tab = (float4 *)(wb + kOffTable);
-    uint32_t *stage = (uint32_t *)(tab + 2 * g.nhkl) + lane;  // full mode
+    float2 *sure = (float2 *)(tab + g.nhkl), *span = sure + g.nhkl;
+    uint32_t *stage = (uint32_t *)(span + g.nhkl) + lane;  // full mode
 
     // ---- set-up: per-slot S*U*B, voxels, zeroed counters
     if (tid < nslot) {
@@ -206,8 +196,8 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
             const OmegaRow d = omega_row(g, b.rot_cs[w0 + wl], b.vpos + 3 * sm.vlist[vl]);
             const RowF r = row_f32(g, d);
             float4 *o = sm.rows + vl * kRowParts * WIN + wl;
-            o[0] = make_float4((float)d.kx, r.ky, r.kz, r.L2);
-            o[WIN] = make_float4(r.cN, r.ay, r.az, r.num);
+            o[0] = make_float4((float)d.kx, r.L2, r.ky, r.kz);
+            o[WIN] = make_float4(r.cN, r.num, r.ay, r.az);
             o[2 * WIN] = make_float4(r.u0, r.v0, r.c, r.s);
             float *kw = (float *)(sm.rows + (vl * kRowParts + 3) * WIN) + wl;
             kw[0] = r.wx;
@@ -278,9 +268,10 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
                 if (ih < g.nhkl) {
                     const float4 gv = gw_of(sf, sm.hk[ih]);
                     const float4 wv = window_f(g, gv);
-                    tab[2 * ih] = gv;
-                    tab[2 * ih + 1] = make_float4(wv.z, wv.w, 0.5f * (wv.x + wv.y),
-                                                  wv.y > wv.x ? 0.25f * (wv.y - wv.x) * (wv.y - wv.x) : -1.0f);
+                    tab[ih] = gv;
+                    sure[ih] = make_float2(wv.z, wv.w);
+                    span[ih] = make_float2(0.5f * (wv.x + wv.y),
+                                           wv.y > wv.x ? 0.25f * (wv.y - wv.x) * (wv.y - wv.x) : -1.0f);
                 }
             }
             __syncwarp();
@@ -305,8 +296,8 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
                 const int ih = (int)(e & 255u), wl = ((int)e >> 8) + pos;
                 int ip = -1;
                 if (valid) {
-                    const float4 gv = tab[2 * ih];
-                    const float2 wv = *(const float2 *)(tab + 2 * ih + 1);
+                    const float4 gv = tab[ih];
+                    const float2 wv = sure[ih];
                     const float4 *o = vr + wl;
                     ip = landing_row3(g, o[0], o[WIN], o[2 * WIN], gv, wv.x, wv.y);
                 }
@@ -379,13 +370,13 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
                         for (int j = 0; j < HPL; ++j) {
                             const int ih = lane + 32 * j;
                             const bool real = ih < g.nhkl;
-                            const float4 gv = tab[real ? 2 * ih : 0];
-                            const float4 wv = tab[real ? 2 * ih + 1 : 1];
+                            const float4 gv = tab[real ? ih : 0];
+                            const float2 wv = span[real ? ih : 0];
                             gx[j] = pack2(gv.x, gv.x);
                             gy[j] = pack2(gv.y, gv.y);
                             gz[j] = pack2(gv.z, gv.z);
-                            mid[j] = pack2(wv.z, wv.z);
-                            const float nh = real ? -wv.w : 1.0f;
+                            mid[j] = pack2(wv.x, wv.x);
+                            const float nh = real ? -wv.y : 1.0f;
                             nh2[j] = pack2(nh, nh);
                             rem[j] = 0;
                         }
