@@ -340,25 +340,26 @@ int run_score(grc_ctx *ctx, const grc::Work &w, int64_t n_trials, bool comp = fa
               unsigned long long *gkey = nullptr, int64_t gsize = 0) {
     TRY(ensure(ctx, ctx->counter, 8 * sizeof(int)));
     TRY(stage_geo(ctx));
-    if (comp) TRY(ensure_bits(ctx));
     if (gkey) CU(cudaMemsetAsync(gkey, 0, sizeof(unsigned long long) * ((n_trials + gsize - 1) / gsize), ctx->stream));
     int launches = 0;
     cudaEvent_t e0 = ctx->timing ? ctx->ev0 : nullptr, e1 = ctx->timing ? ctx->ev1 : nullptr;
     const int64_t round = ctx->force_path == 1 ? 0 : grc::sweep_round_trials(ctx->geo, ctx->num_sms);
     cudaError_t e;
-    // Scan lists whose voxels carry at least a tile of orientations (a sweep tile then meets at
-    // most two voxels) go to the sweep from 1/16 of a round: a one-voxel scan of 2,048
-    // orientations already takes 0.27 ms there against 0.36 ms on the per-trial kernel (8,192:
-    // 0.65 against 1.48 ms), while 1,024 favour the per-trial kernel.  Lists with a voxel per
-    // trial or a few (grow rows, compete, trial lists) keep the half-round rule: there the two
-    // kernels are within 3% of each other up to 16,384 trials.
+    // From a trial per SM on the windowed kernels are faster for every kind of list: a trial per voxel
+    // on Al 1537 x 1001 x 121, 500 voxels 0.098 (per-trial kernel) against 0.080 ms, 9,171 0.40 against
+    // 0.31; 500 voxels with 1-64 candidates 1.86 against 0.32; 256 orientations of one voxel, Al 2048^2
+    // x 361, completeness, 0.127 against 0.088.  Scans of one voxel with medians wait for 1/16 of a
+    // round (4,096 on Fe 1024^2 x 181: 0.579 against 0.230): most of their orientations are wrong, and
+    // on a sparse map, with medians beyond 255 distinct distances, a trial's refine pass costs more
+    // than the scan gains (1,024: 0.168 against 0.127 ms without refine passes, 0.153 against 0.381 with).
     const bool shared_voxels = !w.items && !w.trial_voxel && !w.diag && w.n_or >= 64;
-    const int64_t from = shared_voxels ? (round + 15) / 16 : (round + 1) / 2;
+    const int64_t from = shared_voxels && !comp ? (round + 15) / 16 : ctx->num_sms;
     bool fused_key = false;
     if (round > 0 && (ctx->force_path >= 2 || n_trials >= from)) {
         // projection-window scans (L2-resident map windows) for large trial counts: the warp scan,
         // or the CTA sweep when asked for by grc_set_path(2)
         TRY(ensure(ctx, ctx->rlist, sizeof(int64_t) * n_trials));
+        if (comp) TRY(ensure_bits(ctx));
         grc::ScoreBufs b = bufs(ctx);
         if (comp && gkey) {  // completeness mode folds the first maximum per group in
             b.group_key = gkey;
@@ -1817,9 +1818,9 @@ int batch_enqueue(grc_batch *bt, float *d_out8, float *d_trial_out, int path, in
     w.n_items = m_lim;
     cudaError_t e = cudaSuccess;
     if (T > 0) {
-        // path 1: per-trial kernel; 2: CTA sweep; 3 (and 0 from half a round on): warp scan
+        // path 1: per-trial kernel; 2: CTA sweep; 3 (and 0 from a trial per SM on): warp scan
         const int64_t sr = grc::sweep_round_trials(ctx->geo, ctx->num_sms);
-        const int use = sr == 0 ? 1 : (path != 0 ? path : (T * 2 >= sr ? 3 : 1));
+        const int use = sr == 0 ? 1 : (path != 0 ? path : (T >= ctx->num_sms ? 3 : 1));
         if (use == 2)
             e = grc::launch_sweep(ctx->geo, b, w, T, ctx->num_sms, ctx->stream, e0, e1, launches, slots);
         else if (use == 3)

@@ -141,7 +141,8 @@ __device__ __forceinline__ ScanSmem scan_carve(unsigned char *base, int mode, in
 
 template <int MODE, int HPL, int WIN>
 __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
-    scan_kernel(Geo g, ScoreBufs b, Work w, int64_t round_base, int64_t n_trials, int rows_cap, int slots) {
+    scan_kernel(Geo g, ScoreBufs b, Work w, int64_t round_base, int64_t n_trials, int rows_cap, int slots,
+                int parts_log2) {
     const int64_t cta_base = round_base + (int64_t)blockIdx.x * slots;
     if (cta_base >= n_trials) return;
     const int nslot = (int)min((int64_t)slots, n_trials - cta_base);
@@ -253,13 +254,18 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
             }
         };
 
-        // slots are handed out one at a time, so the warps of a CTA reach the end-of-window
-        // barrier together however unevenly the selected reflections fall on the slots
+        // A slot, or one of the parts its window is cut into where a CTA holds few trials, is handed
+        // out at a time, so the warps of a CTA reach the end-of-window barrier together however
+        // unevenly the selected reflections fall on the slots
+        const int part = WIN >> parts_log2;
         for (;;) {
             int s = 0;
             if (lane == 0) s = atomicAdd(&s_next, 1);
             s = __shfl_sync(kAll, s, 0);
+            const int k0 = (s & ((1 << parts_log2) - 1)) * part, k1 = min(nw, k0 + part);
+            s >>= parts_log2;
             if (s >= nslot) break;
+            if (k0 >= k1) continue;
             // ---- the trial's Gw and window table
             const float *sf = sm.subf + 12 * s;
 #pragma unroll
@@ -359,10 +365,10 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
             constexpr int kSpan = WIN < 32 ? WIN : 32;
             uint32_t rem[HPL];
             bool tested = false;  // rem holds what is left of the span at k
-            int k = 0;
+            int k = k0 & ~(kSpan - 1);
             for (;;) {
                 // leaves this loop when the FP64 queue has no room for a batch, and comes back
-                while (k < nw) {
+                while (k < k1) {
                     if (!tested) {
                         tested = true;
                         uint64_t gx[HPL], gy[HPL], gz[HPL], mid[HPL], nh2[HPL];
@@ -400,7 +406,8 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
                                 rem[j] = __funnelshift_l((uint32_t)d, rem[j], 1);
                             }
                         }
-                        const uint32_t live = nw - k < 32 ? (1u << (nw - k)) - 1u : kAll;
+                        uint32_t live = k1 - k < 32 ? (1u << (k1 - k)) - 1u : kAll;
+                        if (k < k0) live &= kAll << (k0 - k);
 #pragma unroll
                         for (int j = 0; j < HPL; ++j) rem[j] &= live;
                     }
@@ -444,7 +451,7 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
                     tested = false;
                     k += kSpan;
                 }
-                if (k >= nw && fn <= kExactCap - 64) break;
+                if (k >= k1 && fn <= kExactCap - 64) break;
                 __syncwarp();
                 drain_exact(false);
             }
@@ -516,45 +523,49 @@ cudaError_t launch_scan_t(const Geo &g, const ScoreBufs &b, const Work &w, int64
         return rc > sl ? sl : rc;
     };
     size_t offs[kScanParts];
-    using ScanFn = void (*)(Geo, ScoreBufs, Work, int64_t, int64_t, int, int);
+    using ScanFn = void (*)(Geo, ScoreBufs, Work, int64_t, int64_t, int, int, int);
     auto window_kernel = [](int win) -> ScanFn {
-        if constexpr (MODE == kScanComp) {
-            if (win == 128) return scan_kernel<MODE, HPL, 128>;
-            if (win == 64) return scan_kernel<MODE, HPL, 64>;
-        }
+        if (win == 128) return scan_kernel<MODE, HPL, 128>;
+        if (win == 64) return scan_kernel<MODE, HPL, 64>;
         if (win == 32) return scan_kernel<MODE, HPL, 32>;
         return win == 16 ? (ScanFn)scan_kernel<MODE, HPL, 16> : (ScanFn)scan_kernel<MODE, HPL, kScanWinMin>;
     };
-    // the bit-mask window stays within 3/4 of L2 (Al 2048^2 on 126 MB: 128 projections = 67 MB,
-    // fastest; 256 = 134 MB ran 30% slower)
+    // The window's map stays within 3/4 of L2 (Al 2048^2 on 126 MB, bit mask: 128 projections = 67 MB,
+    // fastest; 256 = 134 MB ran 30% slower), or the call touches so few of its pixels that it would
+    // meet few of them again: n_trials * nhkl * window <= 4 * plane (one voxel, full output on 2048^2:
+    // 64 projections against 32 0.339 and 0.348 ms for 4,096 orientations, 0.567 and 0.507 for 9,218).
     int64_t l2_budget = 0;
-    if (MODE == kScanComp) {
-        int dev = 0, l2 = 0;
-        if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) == cudaSuccess)
-            l2_budget = (int64_t)l2 * 3 / 4;
-        else
-            cudaGetLastError();  // no L2 size: windows of at most 32 projections
-    }
-    // Widest window first: up to 128 projections for the bit mask of a seeding scan, 64 for explicit
-    // lists (the refine's grids), 32 for the 8-bit codes, 16 where a tile keeps a row set per trial
-    // (30,000 voxels with 1-64 candidates: 12.6 ms at 16, 14.5 at 32, 15.5 at 8).  Of each, the
-    // most trials per CTA (at most the tile) that keep GRC_SCAN_BLOCKS CTAs within the budget; a
-    // tile below two trials per warp goes on to the next window.
+    int dev = 0, l2 = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) == cudaSuccess)
+        l2_budget = (int64_t)l2 * 3 / 4;
+    else
+        cudaGetLastError();  // no L2 size: windows of at most 32 projections
+    const double reads = (double)n_trials * g.nhkl;
+    // Widest window first: up to 128 projections, 64 for explicit lists of completeness calls (the
+    // refine's grids).  Of each, the most trials per CTA (at most the tile) that keep GRC_SCAN_BLOCKS
+    // CTAs within the budget.  A full-output window above 32 projections is for calls of one round
+    // (2,000 voxels with a trial each, Al 2048^2 x 361: 0.213 ms at 64, 0.225 at 32; 9,171: 0.70 and
+    // 0.68); a tile below one trial per warp, two in completeness mode, goes on to the next window
+    // (30,000 voxels with 1-64 candidates, full output: 11.6 ms at 32 projections and 13 trials, 12.4 at
+    // 16 and 21).
     // A completeness call that a larger tile makes one round takes it.
     if (MODE == kScanComp && !caller_tile && !explicit_voxels &&
         n_trials <= (int64_t)GRC_SCAN_BLOCKS * num_sms * kScanSlots)
         max_slots = kScanSlots;
-    const bool row_per_trial = rows_for(kScanSlotsBulk) == kScanSlotsBulk;
     int win = 0, tile = 0, ctas = GRC_SCAN_BLOCKS;
     for (; ctas >= 1 && !win; --ctas)
         for (int cand : {128, 64, 32, 16, kScanWinMin}) {
-            if (cand > (MODE == kScanFull ? (row_per_trial ? 16 : 32) : explicit_voxels ? 64 : 128)) continue;
-            if (MODE == kScanComp && cand > 32 && (int64_t)cand * b.plane_words * 4 > l2_budget) continue;
-            if (MODE == kScanFull && cand > kScanWinMin && (int64_t)cand * g.plane > 2147483647LL) continue;
+            const int64_t bytes = MODE == kScanComp ? cand * b.plane_words * 4 : cand * g.plane;
+            const bool sparse = reads * cand <= 4.0 * (double)g.plane;
+            if (cand > 32 && bytes > l2_budget && !sparse) continue;
+            if (MODE == kScanComp && explicit_voxels && cand > 64 && !sparse) continue;
+            if (MODE == kScanFull && cand > kScanWinMin && bytes > 2147483647LL) continue;
             int t = max_slots;
             while (t > 0 && ctas * (scan_smem_layout(MODE, g.nhkl, rows_for(t), t, cand, offs) + 1024) > kSmSmemBudget)
                 --t;
-            if (caller_tile ? t < max_slots : t < 2 * kWarps) continue;
+            const bool one_round = (int64_t)t * ctas * num_sms >= n_trials;
+            if (caller_tile ? t < max_slots : !one_round && t < (MODE == kScanComp ? 2 : 1) * kWarps) continue;
+            if (MODE == kScanFull && cand > 32 && !one_round) continue;
             win = cand;
             tile = t;
             break;
@@ -572,6 +583,9 @@ cudaError_t launch_scan_t(const Geo &g, const ScoreBufs &b, const Work &w, int64
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     if (win && per_sm > ctas && ctas >= 1) per_sm = ctas;
     const int64_t grid = (int64_t)per_sm * num_sms;
+    // a trial per warp instead of one to two, over many rounds (the lists above: 11.6 -> 11.3 ms)
+    if (MODE == kScanFull && !caller_tile && tile > kWarps && tile < 2 * kWarps && n_trials > 3 * grid * kWarps)
+        tile = kWarps;
     // rounds of equal size, so that the last is not a sliver
     const int64_t rounds = (n_trials + grid * tile - 1) / (grid * tile);
     int slots = (int)((n_trials + rounds * grid - 1) / (rounds * grid));
@@ -582,13 +596,19 @@ cudaError_t launch_scan_t(const Geo &g, const ScoreBufs &b, const Work &w, int64
     e = allow_smem((const void *)kern, smem);
     if (e != cudaSuccess) return e;
     const int64_t per_round = grid * slots;
+    int parts_log2 = 0;
+    // A window is cut into parts of 32 projections where a CTA holds fewer than two trials per warp,
+    // and of 16 where those would not go round the warps (one voxel, 8 to 256 orientations: 97-125 us
+    // whole, 86-99 at 32, 84-88 at 16).
+    while ((win >> parts_log2) > 32 && slots < 2 * kWarps) ++parts_log2;
+    if (win >= 32 && slots * (win >> 5) < kWarps) ++parts_log2;
     e = cudaMemsetAsync(b.work_counter, 0, 8 * sizeof(int), s);
     if (e != cudaSuccess) return e;
     if (ev0) cudaEventRecord(ev0, s);
     for (int64_t base = 0; base < n_trials; base += per_round) {
         const int64_t left = (n_trials - base + slots - 1) / slots;
         const int gr = (int)(left < grid ? left : grid);
-        kern<<<gr, kThreads, smem, s>>>(g, b, w, base, n_trials, rows_cap, slots);
+        kern<<<gr, kThreads, smem, s>>>(g, b, w, base, n_trials, rows_cap, slots, parts_log2);
         ++*launches;
     }
     if (ev1) cudaEventRecord(ev1, s);
