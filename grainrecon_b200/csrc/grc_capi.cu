@@ -361,7 +361,7 @@ int run_score(grc_ctx *ctx, const grc::Work &w, int64_t n_trials, bool comp = fa
         TRY(ensure(ctx, ctx->rlist, sizeof(int64_t) * n_trials));
         if (comp) TRY(ensure_bits(ctx));
         grc::ScoreBufs b = bufs(ctx);
-        if (comp && gkey) {  // completeness mode folds the first maximum per group in
+        if (gkey) {  // the windowed kernels fold the first maximum per group in
             b.group_key = gkey;
             b.group_size = gsize;
             fused_key = true;

@@ -482,6 +482,14 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
     // ---- finalize
     if constexpr (MODE == kScanFull) {
         for (int s = warp; s < nslot; s += kWarps) hist8_finish(g, b, sm.hist + s * kHistWords, cta_base + s);
+        if (b.group_key) {
+            __syncthreads();
+            for (int base = warp * 32; base < nslot; base += kWarps * 32) {
+                const bool in = base + lane < nslot;
+                const TrialRes r = in ? b.res[cta_base + base + lane] : TrialRes{};
+                fold_group_key(b, in, cta_base + base + lane, r.simu, r.inter);
+            }
+        }
     } else {
         for (int base = warp * 32; base < nslot; base += kWarps * 32) {
             const int s = base + lane;
@@ -545,7 +553,8 @@ cudaError_t launch_scan_t(const Geo &g, const ScoreBufs &b, const Work &w, int64
     // refine's grids).  Of each, the most trials per CTA (at most the tile) that keep GRC_SCAN_BLOCKS
     // CTAs within the budget.  A full-output window above 32 projections is for calls of one round
     // (2,000 voxels with a trial each, Al 2048^2 x 361: 0.213 ms at 64, 0.225 at 32; 9,171: 0.70 and
-    // 0.68); a tile below one trial per warp, two in completeness mode, goes on to the next window
+    // 0.68) or, at 64, for scans whose window's codes stay in L2 (16 voxels x 9,218 orientations, Fe
+    // 1024^2 x 181: 5.25 ms at 32, 5.00 at 64); a tile below one trial per warp, two in completeness mode, goes on to the next window
     // (30,000 voxels with 1-64 candidates, full output: 11.6 ms at 32 projections and 13 trials, 12.4 at
     // 16 and 21).
     // A completeness call that a larger tile makes one round takes it.
@@ -565,7 +574,8 @@ cudaError_t launch_scan_t(const Geo &g, const ScoreBufs &b, const Work &w, int64
                 --t;
             const bool one_round = (int64_t)t * ctas * num_sms >= n_trials;
             if (caller_tile ? t < max_slots : !one_round && t < (MODE == kScanComp ? 2 : 1) * kWarps) continue;
-            if (MODE == kScanFull && cand > 32 && !one_round) continue;
+            if (MODE == kScanFull && cand > 32 && !one_round && (cand > 64 || bytes > l2_budget || t < 2 * kWarps))
+                continue;
             win = cand;
             tile = t;
             break;

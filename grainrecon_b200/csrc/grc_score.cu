@@ -740,6 +740,14 @@ __global__ void __launch_bounds__(kThreads, GRC_SWEEP_BLOCKS) sweep_kernel(Geo g
     // ---- finalize: one warp per slot, exact median from the 8-bit histogram; or the counters
     if constexpr (MODE == kScanFull) {
         for (int s = warp; s < nslot; s += kWarps) hist8_finish(g, b, sm.hist + s * kHist8Words, cta_base + s);
+        if (b.group_key) {
+            __syncthreads();
+            for (int base = warp * 32; base < nslot; base += kWarps * 32) {
+                const bool in = base + lane < nslot;
+                const TrialRes r = in ? b.res[cta_base + base + lane] : TrialRes{};
+                fold_group_key(b, in, cta_base + base + lane, r.simu, r.inter);
+            }
+        }
     } else {
         for (int base = warp * 32; base < nslot; base += kWarps * 32) {
             const int s = base + lane;
