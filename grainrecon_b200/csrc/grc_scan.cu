@@ -5,10 +5,11 @@
 // organised around the warp instead of the CTA:
 //   * a warp takes one trial (slot) of the window at a time and first writes that trial's FP32
 //     Gw table and window thresholds for all reflections into its own shared-memory table;
-//   * 32 projections at a time, each lane tests its reflections against the window and shifts the
-//     sign of the test into a bit mask (6 instructions per pair, no ballot, no store); the set
-//     bits of a mask are runs of consecutive projections, and one entry and one mark bit per run
-//     number the passing pairs, so that a batch of 32 finds its pairs by a population count;
+//   * 32 projections at a time, each lane tests its reflections against the window, two projections
+//     per packed FP32 instruction, and shifts the sign of the test into a bit mask (3 instructions
+//     per pair, no ballot, no store); the set bits of a mask are runs of consecutive projections, and
+//     one entry and one mark bit per run number the passing pairs, so that a batch of 32 finds its
+//     pairs by a population count;
 //   * batches go through the FP32 landing chain with its FP64 band (landing_row3 / landing_exact).
 //     Lanes hold consecutive projections of a few reflections: their omega rows are consecutive
 //     16-byte words in shared memory, their Gw words broadcasts;
@@ -17,15 +18,16 @@
 //     which a third miss L2;
 //   * ambiguous items keep their trial in the warp's FP64 queue, drained outside the batch loop: a
 //     call inside it cost 12 spill reloads per batch.
-// What bounds it (FCC Al 2048^2 x 361, completeness): issue (69 % of slots, 28.3 k warp instructions
-// per trial) and the shared-memory / L1 pipe (78 % of its wavefronts: 12 of a batch's 56 are its
-// rows, some 20 its gather) together.  Against one ballot and one queue store per (projection, slot)
-// and 64-byte rows (40.6 k instructions): 64 seeds x 32,768 orientations 97.4 -> 73.2 ms, four
-// columns (16 seeds) 32.6 (CTA sweep) -> 25.6 ms.  Numbering the pairs projection-major instead
-// (masks transposed across the warp, better shared rows) ran 82.0 ms: its Gw words conflict.  Four
-// CTAs per SM (64 registers) ran 114 ms.
-// Windows: up to 32 projections of 8-bit codes (full mode), up to 128 of the bit mask
-// (completeness mode), each within the limits of shared memory and L2 (launch_scan_t).
+// What bounds it (FCC Al 2048^2 x 361, completeness): issue (68 % of slots, 24.9 k warp instructions
+// per trial) and the shared-memory / L1 pipe (80 % of its wavefronts: 12 of a batch's 31 are its
+// rows, 13 its gather) together.  64 seeds x 32,768 orientations: one ballot and one queue store per
+// (projection, slot) and 64-byte rows (40.6 k instructions) 97.4 ms; bit masks and runs 73.2; the
+// test two projections per instruction 70.0; landings in packed pairs, separate tables 68.8.
+// Four columns (16 seeds), before the last two: 32.6 (CTA sweep) -> 25.6 ms.  Numbering the pairs
+// projection-major instead (masks transposed across the warp, better shared rows) ran 82.0 ms: its
+// Gw words conflict.  Four CTAs per SM (64 registers) ran 114 ms.  Rows of 10 numbers (kx and L2
+// from ky and kz) ran 71.2: two wavefronts fewer do not pay for six instructions more.
+// Windows: up to 128 projections within the limits of shared memory and L2 (launch_scan_t).
 // The decisions are those of the sweep and of the oracle: same prefilter margins, same FP32
 // algebra and band, same FP64 path.
 #include <cuda_runtime.h>

@@ -1,5 +1,5 @@
 """Spot-centroid fits on the GPU: synthetic matched spots, Levenberg-Marquardt with
-tangent-derived Jacobians, and the forward-only Nelder-Mead (fminsearchbnd) baseline.
+adjoint Jacobians, and the forward-only Nelder-Mead (fminsearchbnd) baseline.
 
 Replaces the fminsearchbnd fits of fit_grain_COM.m:5-88 / fit_OR_constrain_* (per grain:
 Rodrigues vector + centre) and GrainMapping_fit_geo.m / L_shift_tilt_fitting.m:23-50

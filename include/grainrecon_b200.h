@@ -438,8 +438,9 @@ int grc_fit_spot_fill(grc_ctx *ctx, const double *geo10, const double *d_grains,
                       const int64_t *d_offsets, int32_t *d_grain, int32_t *d_iw, int32_t *d_ih, double *d_uv);
 /*
  * Residuals (model - measured, 2 per spot) and Jacobian rows d(u,v)/d(params) (2*K per
- * spot, u row then v row) by hand-propagated FP64 tangents; mode 0: K = 6 grain parameters,
- * mode 1: K = 10 geometry parameters.  The loss gradient is J^T r.  A spot that leaves the
+ * spot, u row then v row) by FP64 derivatives taken backwards through the landing; mode 0:
+ * K = 6 grain parameters, mode 1: K = 10 geometry parameters.  The loss gradient is J^T r.  A
+ * spot that leaves the
  * wavelength window or the detector gets NaN residuals.
  */
 int grc_centroid_residual_adjoint(grc_ctx *ctx, int mode, const double *geo10, const double *d_grains,
@@ -494,10 +495,10 @@ int grc_last_stats(grc_ctx *ctx, grc_stats *out);
 int grc_set_timing(grc_ctx *ctx, int enable);
 /*
  * Scoring kernel selection: 0 = by size (default: the projection-window warp scan, which keeps
- * the map windows L2-resident and runs one trial per warp at a time, once a call holds 1/16 of a
- * round of trials -- 1,776 on 148 SMs -- when each voxel carries at least 64 orientations, or
- * half a round otherwise; the CTA sweep for full-output calls of more than two rounds on
- * geometries of fewer than 5,000 (projection, reflection) pairs; the per-trial kernel below those
+ * the map windows L2-resident and runs one trial per warp at a time, once a call holds a trial per
+ * SM -- scans of one voxel with medians 1/16 of a round of trials, 1,776 on 148 SMs; the CTA sweep
+ * for full-output calls of more than two rounds on geometries of fewer than 5,000 (projection,
+ * reflection) pairs; the per-trial kernel below those
  * sizes), 1 = always the per-trial kernel,
  * 2 = always the CTA sweep (the same windows with the trials of a CTA mixed in its batches),
  * 3 = always the warp scan.  Results are identical; only speed differs.  Batches (grc_batch_*)
