@@ -18,8 +18,8 @@
 //     which a third miss L2;
 //   * ambiguous items keep their trial in the warp's FP64 queue, drained outside the batch loop: a
 //     call inside it cost 12 spill reloads per batch.
-// What bounds it (FCC Al 2048^2 x 361, completeness): issue (68 % of slots, 24.9 k warp instructions
-// per trial) and the shared-memory / L1 pipe (80 % of its wavefronts: 12 of a batch's 31 are its
+// What bounds it (FCC Al 2048^2 x 361, completeness): issue (66 % of slots, 25.3 k warp instructions
+// per trial) and the shared-memory / L1 pipe (79 % of its wavefronts: 12 of a batch's 31 are its
 // rows, 13 its gather) together.  64 seeds x 32,768 orientations: one ballot and one queue store per
 // (projection, slot) and 64-byte rows (40.6 k instructions) 97.4 ms; bit masks and runs 73.2; the
 // test two projections per instruction 70.0; landings in packed pairs, separate tables 68.8.
