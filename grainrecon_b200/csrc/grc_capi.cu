@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "grainrecon_b200.h"
+#include "grc_band.h"
 #include "grc_fit.h"
 #include "grc_internal.h"
 
@@ -155,6 +156,11 @@ void apply_options(grc_ctx *ctx) {
     g.lo4pif = (float)(g.lmin * 0.25 / 3.14159265358979323846);
     g.hi4pif = (float)(g.lmax * 0.25 / 3.14159265358979323846);
     g.cbmaxf = (float)g.cbmax;
+    const grc::Fp32Limits lim = grc::fp32_limits(g);
+    g.half_u = lim.half_u;
+    g.half_v = lim.half_v;
+    g.sin_sure = lim.sin_sure;
+    g.reach2f = (float)lim.reach2;
     refresh_hit(ctx);
 }
 
@@ -215,6 +221,16 @@ int set_geometry(grc_ctx *ctx, const float *S, const float *B, const float *hkl,
     }
     std::vector<double> h(3 * nhkl);
     for (int i = 0; i < 3 * nhkl; ++i) h[i] = hkl[i];
+    double s2 = 0;
+    for (int i = 0; i < 9; ++i) s2 += g.S[i] * g.S[i];
+    for (int i = 0; i < nhkl; ++i) {
+        double b2 = 0;
+        for (int r = 0; r < 3; ++r) {
+            const double b = g.B[3 * r] * h[3 * i] + g.B[3 * r + 1] * h[3 * i + 1] + g.B[3 * r + 2] * h[3 * i + 2];
+            b2 += b * b;
+        }
+        g.gmax = std::max(g.gmax, std::sqrt(b2 * s2 / 3.0));
+    }
     TRY(ensure(ctx, ctx->rot_cs, sizeof(double2) * nrot));
     TRY(ensure(ctx, ctx->hkl, sizeof(double) * 3 * nhkl));
     CU(cudaMemcpyAsync(ctx->rot_cs.p, cs.data(), sizeof(double2) * nrot, cudaMemcpyHostToDevice, ctx->stream));
@@ -1548,6 +1564,10 @@ int grc_pair_spots(grc_ctx *ctx, const double *d_pos, const double *d_q, int64_t
                       (const double *)ctx->sp_yz.p, ncy, ncz};
     CU(cudaMemsetAsync(ctx->pcount.p, 0, sizeof(unsigned long long), s));
     TRY(stage_geo(ctx));
+#ifdef GRC_AUDIT
+    TRY(ensure(ctx, ctx->counter, 8 * sizeof(int)));
+    CU(cudaMemsetAsync(ctx->counter.p, 0, 8 * sizeof(int), s));
+#endif
     grc::PairUnits u{};
     u.count = (int64_t *)ctx->pr_units.p;
     u.seg = u.count + units;

@@ -32,18 +32,13 @@ struct __align__(16) RowF {
 };
 static_assert(sizeof(RowF) == 64, "RowF layout");
 
-// Pixel-rounding ambiguity band of the FP32 landing chain.  Its error against the
-// FP64 chain stays below 1.4e-3 px on the 1024^2 / 2048^2 geometries (measured over
-// 3.4e5 landings); landings closer than this to a half-pixel boundary are recomputed
-// in FP64, so every decision equals the FP64 one.  A build with -DGRC_AUDIT re-decides
-// every FP32 decision in FP64 (CTA sweep): at 0.003 px it found no disagreement in
-// 1.72e10 decisions (FCC Al 2048^2 x 361 and BCC Fe 1024^2 x 181 scans, 64 seeds x 32,768
-// orientations each), at 0.001 px two in 1.7e9; the band keeps a third above the audited
-// 0.003 px.
-#ifndef GRC_AMBIG_PX
-#define GRC_AMBIG_PX 0.004f
-#endif
-constexpr float kAmbigPx = GRC_AMBIG_PX;
+// Pixel-rounding ambiguity band of the FP32 landing chains: landings closer to a half-pixel boundary
+// than the geometry's band (grc_band.h; Geo half_u, half_v hold half a pixel less it) are
+// recomputed in FP64, so every decision equals the FP64 one.  A build with -DGRC_AUDIT re-decides
+// every FP32 decision of the scans and of pairing in FP64; -DGRC_AMBIG_PX narrows all bands in
+// proportion.  FCC Al 2048^2 x 361 and BCC Fe 1024^2 x 181 (band 0.004 px), 64 seeds x 32,768
+// orientations each: landing_fp32 (CTA sweep) at 0.003 px no disagreement in 1.72e10 decisions, at
+// 0.001 px two in 1.7e9; landing_row3 (warp scan) at 0.002 px none in 5.8e9.
 
 __device__ __forceinline__ size_t align16(size_t x) { return (x + 15) & ~size_t(15); }
 
@@ -74,14 +69,21 @@ __device__ __forceinline__ OmegaRow omega_row(const Geo &g, const double2 cs, co
     return r;
 }
 
-// FP32 row from the FP64 one (the folded constants are formed in FP64 and rounded once).
-__device__ __forceinline__ RowF row_f32(const Geo &g, const OmegaRow &r) {
+// Whether a voxel lies within the distance that the FP32 band was formed for.
+__device__ __forceinline__ bool in_reach(const Geo &g, const double *__restrict__ vp) {
+    const float x = (float)vp[0], y = (float)(vp[1] - g.rao), z = (float)vp[2];
+    return x * x + y * y + z * z <= g.reach2f;
+}
+
+// FP32 row from the FP64 one (the folded constants are formed in FP64 and rounded once).  A voxel
+// out of reach gets no u: its landings are all decided in FP64.
+__device__ __forceinline__ RowF row_f32(const Geo &g, const OmegaRow &r, bool reach) {
     RowF f;
     f.cN = (float)(g.R[0] * r.ax);
     f.ky = (float)r.ky; f.kz = (float)r.kz; f.L2 = (float)r.L2;
     f.cY = (float)(g.R[1] * r.ax * g.rpxy);
     f.ay = (float)r.ay; f.az = (float)r.az; f.num = (float)r.num;
-    f.u0 = (float)(g.dety0 - r.r2d * g.rpxy);
+    f.u0 = reach ? (float)(g.dety0 - r.r2d * g.rpxy) : CUDART_NAN_F;
     f.v0 = (float)(g.detz0 - r.r3d * g.rpxz);
     f.c = (float)r.c; f.s = (float)r.s;
     f.wx = (float)(r.c * r.kx + r.s * r.ky);
@@ -94,7 +96,9 @@ __device__ __forceinline__ RowF row_f32(const Geo &g, const OmegaRow &r) {
 // Omega table of one voxel in shared memory (all threads of the CTA).
 __device__ void build_rows(const Geo &g, const double2 *__restrict__ rot_cs, const double *__restrict__ vp,
                            RowF *rows) {
-    for (int iw = threadIdx.x; iw < g.nrot; iw += blockDim.x) rows[iw] = row_f32(g, omega_row(g, rot_cs[iw], vp));
+    const bool reach = in_reach(g, vp);
+    for (int iw = threadIdx.x; iw < g.nrot; iw += blockDim.x)
+        rows[iw] = row_f32(g, omega_row(g, rot_cs[iw], vp), reach);
 }
 
 // SUB = S*U*B (FP64, 9 values) of one trial.
@@ -184,7 +188,8 @@ __device__ __noinline__ int64_t landing_exact(const Geo *__restrict__ gd, const 
 // Window thresholds of one reflection on t = -(k_w . Gw) = |G|^2 lambda / (4 pi):
 // lambda in (lambda_min, lambda_max) and cos(beta) > cos(beta_max).  Returned as
 // (lo, hi) = the interval widened by the FP32 margin (prefilter) and (lo_in, hi_in)
-// = narrowed by it (inside, the FP32 decision is certain).
+// = narrowed by it and by the Bragg angle up to which the band holds (inside, the FP32 decision is
+// certain).
 __device__ __forceinline__ float4 window_of(const Geo &g, float G_f) {
     const double G = G_f, G2 = G * G;
     const double inv4pi = 0.25 / CUDART_PI;
@@ -192,7 +197,7 @@ __device__ __forceinline__ float4 window_of(const Geo &g, float G_f) {
     if (g.cbmax > -1.0) hi = fmin(hi, -g.cbmax * G);
     lo = fmax(lo, 0.0);
     const double m = 1e-5 * G;  // >> FP32 error of k_w . G (~4e-7 |G|)
-    return make_float4((float)(lo - m), (float)(hi + m), (float)(lo + m), (float)(hi - m));
+    return make_float4((float)(lo - m), (float)(hi + m), (float)(lo + m), fminf((float)(hi - m), g.sin_sure * G_f));
 }
 
 // MUFU reciprocal and reciprocal square root without the denormal scaling code around them: every
@@ -250,7 +255,7 @@ __device__ __forceinline__ int pixel_of(const Geo &g, uint64_t uv, bool certain)
     constexpr float kRound = 12582912.0f;
     const uint64_t t2 = add2(uv, pack2(kRound, kRound)), r2 = add2(t2, pack2(-kRound, -kRound));
     const float2 t = unpack2(t2), r = unpack2(r2), d = unpack2(fma2(r2, pack2(-1.0f, -1.0f), uv));
-    certain = certain & (fabsf(d.x) <= 0.5f - kAmbigPx) & (fabsf(d.y) <= 0.5f - kAmbigPx);
+    certain = certain & (fabsf(d.x) <= g.half_u) & (fabsf(d.y) <= g.half_v);
     const uint32_t iu = (uint32_t)(__float_as_int(t.x) - 0x4B400001), iv = (uint32_t)(__float_as_int(t.y) - 0x4B400001);
     bool in = (iu < (uint32_t)g.detysize) & (iv < (uint32_t)g.detzsize);  // 0-based pixel
     if (g.beam_stop) in = in & !((r.x >= g.bsy0f) & (r.x <= g.bsy1f) & (r.y >= g.bsz0f) & (r.y <= g.bsz1f));
@@ -288,7 +293,7 @@ __device__ __forceinline__ int landing_fp32(const Geo &g, const RowF &r, const f
     const float v = r.v0 - f * (r.cZ + g.Ryf.y * Ky + g.Rzf.y * Kz);
     if (!(fabsf(u) < 2e6f && fabsf(v) < 2e6f)) {  // detectors have at most 10^6 pixels per side
         // far off the detector (or NaN): certain rejection only for finite values
-        return (isfinite(u) && isfinite(v)) ? -1 : -2;
+        return (isfinite(u) && isfinite(v) && g.half_u > 0.0f) ? -1 : -2;
     }
     // nearest integer by the 1.5*2^23 addition (|u|, |v| < 2^22 here): the sum's low mantissa
     // bits hold the rounded value, read back as an integer without a conversion instruction.
@@ -297,7 +302,7 @@ __device__ __forceinline__ int landing_fp32(const Geo &g, const RowF &r, const f
     constexpr float kRound = 12582912.0f;
     const float tu = __fadd_rn(u, kRound), tv = __fadd_rn(v, kRound);
     const float ru = __fsub_rn(tu, kRound), rv = __fsub_rn(tv, kRound);
-    if (fabsf(u - ru) > 0.5f - kAmbigPx || fabsf(v - rv) > 0.5f - kAmbigPx) return -2;
+    if (fabsf(u - ru) > g.half_u || fabsf(v - rv) > g.half_v) return -2;
     const int iu = __float_as_int(tu) - 0x4B400000, iv = __float_as_int(tv) - 0x4B400000;
     if (!(iu >= 1 && iu <= g.detysize && iv >= 1 && iv <= g.detzsize)) return -1;
     if (ru >= g.bsy0f && ru <= g.bsy1f && rv >= g.bsz0f && rv <= g.bsz1f) return -1;
@@ -346,7 +351,7 @@ __device__ __forceinline__ float4 window_f(const Geo &g, const float4 gv) {
     if (g.cbmaxf > -1.0f) hi = fminf(hi, -g.cbmaxf * G);
     lo = fmaxf(lo, 0.0f);
     const float m = 1e-5f * G;
-    return make_float4(lo - m, hi + m, lo + m, hi - m);
+    return make_float4(lo - m, hi + m, lo + m, fminf(hi - m, g.sin_sure * G));
 }
 
 // Result of one trial from its 8-bit code histogram (256 u16 bins in 128 words; bin 255 counts the

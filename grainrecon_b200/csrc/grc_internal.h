@@ -22,6 +22,7 @@ struct Geo {
     double rpxy, rpxz;       // 1 / pixel sizes
     double lmin, lmax;       // wavelength window [A]
     double cbmax;            // cos((90+4*thetamax) deg), or -2 when that angle is >= 180 deg
+    double gmax;             // longest |S U B h| of an orthonormal U
     double bsy0, bsy1, bsz0, bsz1;
     double S[9], B[9], R[9]; // row-major
     // FP32 copies for the fast landing chain
@@ -30,6 +31,8 @@ struct Geo {
     // and R[0] K_x times Raf = {R[1]/(R[0] pxy), R[2]/(R[0] pxz)}
     float2 Ryf, Rzf, Raf;
     float dety0f, detz0f, rpxyf, rpxzf;
+    float half_u, half_v;    // FP32 landings: certain up to here from a pixel's centre (grc_band.h)
+    float sin_sure, reach2f; // and up to this sin(theta) and squared distance of the voxel from the rotation axis' origin
     float bsy0f, bsy1f, bsz0f, bsz1f;
     int beam_stop;           // 0 when the beam stop covers no pixel of the detector
     float lo4pif, hi4pif, cbmaxf;   // lambda_min/(4 pi), lambda_max/(4 pi), cos(beta_max)

@@ -172,6 +172,7 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
             sm.subf[12 * tid + i] = (float)SUB[i];
         }
         sm.vglob[tid] = v;
+        sm.vloc[tid] = in_reach(g, b.vpos + 3 * v) ? 0 : 1;
     }
     for (int i = tid; i < slots * (MODE == kScanFull ? kHistWords : 1); i += kThreads) sm.hist[i] = 0;
     for (int i = tid; i < g.nhkl; i += kThreads)
@@ -181,7 +182,8 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
     if (tid == 0) {
         int nv = 0;
         for (int s = 0; s < nslot; ++s) {
-            if (s == 0 || sm.vglob[s] != sm.vglob[s - 1]) sm.vlist[nv++] = sm.vglob[s];
+            // ~voxel: out of reach of the FP32 landings
+            if (s == 0 || sm.vglob[s] != sm.vglob[s - 1]) sm.vlist[nv++] = sm.vloc[s] ? ~sm.vglob[s] : sm.vglob[s];
             sm.vloc[s] = nv - 1;
         }
         s_nv = nv;
@@ -196,8 +198,9 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
         // ---- omega rows of this window for every voxel of the round
         for (int i = tid; i < nv * nw; i += kThreads) {
             const int vl = i / nw, wl = i - vl * nw;
-            const OmegaRow d = omega_row(g, b.rot_cs[w0 + wl], b.vpos + 3 * sm.vlist[vl]);
-            const RowF r = row_f32(g, d);
+            const int64_t v = sm.vlist[vl];
+            const OmegaRow d = omega_row(g, b.rot_cs[w0 + wl], b.vpos + 3 * (v < 0 ? ~v : v));
+            const RowF r = row_f32(g, d, v >= 0);
             float4 *o = sm.rows + vl * kRowParts * WIN + wl;
             o[0] = make_float4((float)d.kx, r.L2, r.ky, r.kz);
             o[WIN] = make_float4(r.cN, r.num, r.ay, r.az);

@@ -561,6 +561,7 @@ __global__ void __launch_bounds__(kThreads, GRC_SWEEP_BLOCKS) sweep_kernel(Geo g
             sm.subf[12 * tid + i] = (float)SUB[i];
         }
         sm.vglob[tid] = v;
+        sm.vloc[tid] = in_reach(g, b.vpos + 3 * v) ? 0 : 1;
     }
     for (int i = tid; i < slots * (MODE == kScanFull ? kHist8Words : 1); i += kThreads) sm.hist[i] = 0;
     for (int i = tid; i < g.nhkl; i += kThreads)
@@ -569,7 +570,8 @@ __global__ void __launch_bounds__(kThreads, GRC_SWEEP_BLOCKS) sweep_kernel(Geo g
     if (tid == 0) {
         int nv = 0;
         for (int s = 0; s < nslot; ++s) {
-            if (s == 0 || sm.vglob[s] != sm.vglob[s - 1]) sm.vlist[nv++] = sm.vglob[s];
+            // ~voxel: out of reach of the FP32 landings
+            if (s == 0 || sm.vglob[s] != sm.vglob[s - 1]) sm.vlist[nv++] = sm.vloc[s] ? ~sm.vglob[s] : sm.vglob[s];
             sm.vloc[s] = nv - 1;
         }
         s_nv = nv;
@@ -623,7 +625,8 @@ __global__ void __launch_bounds__(kThreads, GRC_SWEEP_BLOCKS) sweep_kernel(Geo g
         // ---- omega rows of this window for every voxel of the round
         for (int i = tid; i < nv * nw; i += kThreads) {
             const int vl = i / nw, wl = i - vl * nw;
-            sm.rows[vl * nwin + wl] = row_f32(g, omega_row(g, b.rot_cs[w0 + wl], b.vpos + 3 * sm.vlist[vl]));
+            const int64_t v = sm.vlist[vl];
+            sm.rows[vl * nwin + wl] = row_f32(g, omega_row(g, b.rot_cs[w0 + wl], b.vpos + 3 * (v < 0 ? ~v : v)), v >= 0);
         }
         if (tid == 0) s_next = 0;
         __syncthreads();
@@ -1064,7 +1067,8 @@ __global__ void __launch_bounds__(kPairThreads, 6) pair_find_k(Geo g, ScoreBufs 
         const int iw0 = (int)(unit - t * n_chunk) * unit_rows, nw = min(unit_rows, g.nrot - iw0), P = nw * nh;
         const double *vp = b.vpos + 3 * t;
         __syncthreads();  // the previous unit's tables are no longer read
-        for (int i = tid; i < nw; i += kPairThreads) rows[i] = row_f32(g, omega_row(g, b.rot_cs[iw0 + i], vp));
+        const bool reach = in_reach(g, vp);
+        for (int i = tid; i < nw; i += kPairThreads) rows[i] = row_f32(g, omega_row(g, b.rot_cs[iw0 + i], vp), reach);
         build_gw(g, b.hkl, b.U + 9 * t, gw, win, sub);
         for (int i = tid; i < P; i += kPairThreads) spot[i] = -1;
         if (tid == 0) s_hits = s_undecided = 0;
@@ -1101,6 +1105,13 @@ __global__ void __launch_bounds__(kPairThreads, 6) pair_find_k(Geo g, ScoreBufs 
             const int wl = (int)(it >> 8), ih = (int)(it & 255u);
             int ip = -1;
             if (valid) ip = landing_fp32(g, rows[wl], gw[ih], win[ih].z, win[ih].w);
+#ifdef GRC_AUDIT
+            if (valid && ip != -2) {
+                const int64_t r64 = landing_exact(b.geo, b.rot_cs, vp, b.hkl, sub, iw0 + wl, ih);
+                atomicAdd((unsigned long long *)(b.work_counter + 6), 1ull);
+                if ((r64 >= 0 ? (int)(r64 - (int64_t)(iw0 + wl) * g.plane) : -1) != ip) atomicAdd(b.work_counter + 5, 1);
+            }
+#endif
             join(undecided, &s_undecided, wl * nh + ih, ip == -2);
             found(wl * nh + ih, wl, ip);
         };
