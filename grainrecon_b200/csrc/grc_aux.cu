@@ -774,6 +774,7 @@ cudaError_t encode_map(const float *d_map, int64_t n, cudaStream_t s, MapCodes *
     MapCodes out{};
     void *tmp = nullptr;
     cudaError_t e;
+    bool shared = false;  // buffers of the resident map are being written
     *bad_nan = 0;
 #define CK(x)                                       \
     do {                                            \
@@ -820,6 +821,8 @@ cudaError_t encode_map(const float *d_map, int64_t n, cudaStream_t s, MapCodes *
         CK(take_buffer((void **)&out.codes8, &out.cap_codes8, resident->codes8, resident->cap_codes8,
                        ((size_t)n + 3) & ~size_t(3)));
         CK(take_buffer(&out.codes, &out.cap_codes, resident->codes, resident->cap_codes, (size_t)n * (c16 ? 2 : 4)));
+        shared = (out.codes && out.codes == resident->codes) || (out.codes8 && out.codes8 == resident->codes8) ||
+                 (out.vals && out.vals == resident->vals);
         values_k<<<blocks_for(nw), kB, 0, s>>>(bitmap, prefix, half_of, nw, pairs, out.vals);
         if (c16)
             codes_k<uint16_t><<<blocks, kB, 0, s>>>(d_map, n, halves, before, pairs, (uint16_t *)out.codes, out.codes8);
@@ -840,6 +843,7 @@ failed:
     if (out.codes != resident->codes) cudaFree(out.codes);
     if (out.codes8 != resident->codes8) cudaFree(out.codes8);
     if (out.vals != resident->vals) cudaFree(out.vals);
+    if (shared) resident->release();  // partly overwritten: no map is left
     return e;
 }
 

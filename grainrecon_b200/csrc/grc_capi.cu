@@ -247,7 +247,10 @@ int upload_device_map(grc_ctx *ctx, const float *d_map, int64_t dz, int64_t dy, 
     const int64_t n = dz * dy * nrot;
     int bad = 0;
     cudaError_t e = grc::encode_map(d_map, n, ctx->stream, &ctx->mc, ctx->map_ws, &bad);
-    if (e != cudaSuccess) return fail(ctx, GRC_ECUDA, "distance-map coding: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        if (!ctx->mc.codes) ctx->has_masks = ctx->bits_ok = false;  // failed while it wrote the map's buffers
+        return fail(ctx, GRC_ECUDA, "distance-map coding: %s", cudaGetErrorString(e));
+    }
     if (bad) return fail(ctx, GRC_EINVAL, "distance map holds NaN values");
     // from here the codes are the new map's: without its values there is no map
     ctx->has_masks = false;

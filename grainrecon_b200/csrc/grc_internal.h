@@ -205,8 +205,9 @@ struct MapCodes {
     void release();
 };
 // Encodes d_map (n floats) into *resident, whose buffers are reused where they fit.  A map with NaN
-// values (*bad_nan) or a failed call leaves *resident valid; nothing of it is written before the map is
-// known to be good and every buffer allocated.  ws: two scratches.
+// values (*bad_nan), or a call that fails before the map is known to be good and every buffer
+// allocated, leaves *resident as it is; one that fails after that, with reused buffers partly
+// written, leaves it empty.  ws: two scratches.
 cudaError_t encode_map(const float *d_map, int64_t n, cudaStream_t s, MapCodes *resident, Scratch *ws, int *bad_nan);
 
 // Synthetic-data kernels.
