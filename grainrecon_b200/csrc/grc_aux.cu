@@ -776,6 +776,11 @@ cudaError_t encode_map(const float *d_map, int64_t n, cudaStream_t s, MapCodes *
     cudaError_t e;
     bool shared = false;  // buffers of the resident map are being written
     *bad_nan = 0;
+    if (n <= 0) {  // no pixel, no value
+        resident->n_distinct = 0;
+        resident->code_bits = 0;
+        return cudaSuccess;
+    }
 #define CK(x)                                       \
     do {                                            \
         if ((e = (x)) != cudaSuccess) goto failed;  \

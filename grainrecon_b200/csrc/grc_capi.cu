@@ -255,7 +255,7 @@ int upload_device_map(grc_ctx *ctx, const float *d_map, int64_t dz, int64_t dy, 
     // from here the codes are the new map's: without its values there is no map
     ctx->has_masks = false;
     std::vector<float> hv((size_t)ctx->mc.n_distinct);
-    e = cudaMemcpy(hv.data(), ctx->mc.vals, sizeof(float) * hv.size(), cudaMemcpyDeviceToHost);
+    if (!hv.empty()) e = cudaMemcpy(hv.data(), ctx->mc.vals, sizeof(float) * hv.size(), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return fail(ctx, GRC_ECUDA, "value table copy: %s", cudaGetErrorString(e));
     ctx->bits_ok = false;  // packed again from the new codes when first needed
     ctx->map_key = 0;      // an upload that came without a key

@@ -46,3 +46,16 @@ def test_a_failed_upload_leaves_a_whole_map_or_none(fake, ctx, at, left):
     ctx._dev(ctx.L.grc_upload_masks, d, 32, 64, 2)
     assert resident(ctx) == (5, 32, 64, 2)
     assert fake.stray() == 0
+
+
+@pytest.mark.parametrize("dims", [(0, 32, 2), (64, 0, 2), (64, 32, 0), (-5, 1, 1), (-1, -1, -3)])
+def test_an_empty_device_map(fake, ctx, dims):
+    """Accepted by grc_upload_masks as a map without values; nothing is read or copied for it."""
+    fake.reset()
+    d = fake.alloc(64)
+    assert ctx.L.grc_upload_masks(ctx.h, d, *dims) == _lib.GRC_OK
+    assert fake.stray() == 0 and fake.launched() == []
+    assert resident(ctx) == (0, *dims)
+    code_map(fake, 4)
+    ctx._dev(ctx.L.grc_upload_masks, fake.alloc(4 * 64 * 32 * 2), 64, 32, 2)
+    assert resident(ctx) == (4, 64, 32, 2)
