@@ -385,6 +385,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 3 : 1) grain_lm_k(Fi
     __shared__ Beam e;
     __shared__ double s_g[6], s_ub[9];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    bool moved = false;  // thread 0: the step changed a parameter
     if (t == 0) make_beam(geo10, e);
     for (int64_t gi = blockIdx.x; gi < n_grains; gi += gridDim.x) {
         __syncthreads();
@@ -425,7 +426,12 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 3 : 1) grain_lm_k(Fi
         if (threadIdx.x == 0) {
             double x[6] = {0, 0, 0, 0, 0, 0};
             const bool ok = s_ne[28] >= 6 && lm_solve<6>(s_ne, s_ne + 21, lambda[gi], x);
-            for (int k = 0; k < 6; ++k) s_g[k] += ok ? x[k] : 0.0;
+            moved = false;
+            for (int k = 0; k < 6; ++k) {
+                const double to = s_g[k] + (ok ? x[k] : 0.0);
+                moved |= to != s_g[k];
+                s_g[k] = to;
+            }
             make_ub(fx, s_g, s_ub);
         }
         __syncthreads();
@@ -439,7 +445,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 3 : 1) grain_lm_k(Fi
         }
         block_sum<1>(cost, scratch);
         if (threadIdx.x == 0) {
-            if (cost[0] < now) {
+            if (moved && cost[0] < now) {  // the two sums of one point differ by rounding
                 for (int k = 0; k < 6; ++k) grains[6 * gi + k] = s_g[k];
                 lambda[gi] = fmax(lambda[gi] * 0.1, 1e-9);
                 if (now - cost[0] > 1e-9 * now) atomicAdd(improved, 1);
@@ -703,7 +709,9 @@ __global__ void geo_lm_accept_k(double *starts, const double *trial, const doubl
     const int st = blockIdx.x * blockDim.x + threadIdx.x;
     if (st >= n) return;
     const double now = ne[st * kNE10 + 65] + 1e6 * ((double)n_spots - ne[st * kNE10 + 66]);
-    if (cost_trial[2 * st] < now) {
+    bool moved = false;  // the two sums of one point differ by rounding
+    for (int k = 0; k < 10; ++k) moved |= trial[10 * st + k] != starts[10 * st + k];
+    if (moved && cost_trial[2 * st] < now) {
         for (int k = 0; k < 10; ++k) starts[10 * st + k] = trial[10 * st + k];
         lambda[st] = fmax(lambda[st] * 0.1, 1e-9);
         if (now - cost_trial[2 * st] > 1e-9 * now) atomicAdd(improved, 1);
