@@ -104,7 +104,7 @@ __device__ __forceinline__ bool land_spot(const FitFixed &fx, const Beam &e, con
     const double x = (kx * Gx + ky * Gy + kz * Gz) * rG;
     const double lam = -4.0 * CUDART_PI * rG * x;
     if (strict && !(x < 0.0 && x > fx.cbmax && lam > fx.lmin && lam < fx.lmax)) return false;
-    const double q = 1.0 - x * x, rct = rsqrt(q), ct = q * rct;
+    const double q = 1.0 - x * x, rct = rsqrt(q), ct = q == 0.0 ? 0.0 : q * rct;  // 0: straight back
     const double s2 = -2.0 * x * ct, c2 = 1.0 - 2.0 * x * x;
     const double cph = gy * ky + gz * kz, p = 1.0 - cph * cph, rsph = rsqrt(p), sph = p * rsph;
     const double rs = 1.0 / (sph * c2 - cph * s2);  // 1 / sin(phi - tau)
