@@ -73,6 +73,7 @@ int fail(grc_ctx *c, int code, const char *fmt, ...) {
     vsnprintf(buf, sizeof buf, fmt, ap);
     va_end(ap);
     if (c) c->err = buf;
+    if (code == GRC_ECUDA) cudaGetLastError();  // reported here: the next call's launch checks start clean
     return code;
 }
 
