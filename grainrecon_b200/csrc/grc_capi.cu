@@ -375,11 +375,18 @@ int run_score(grc_ctx *ctx, const grc::Work &w, int64_t n_trials, bool comp = fa
     const bool shared_voxels = !w.items && !w.trial_voxel && !w.diag && w.n_or >= 64;
     const int64_t from = shared_voxels && !comp ? (round + 15) / 16 : ctx->num_sms;
     bool fused_key = false;
-    if (round > 0 && (ctx->force_path >= 2 || n_trials >= from)) {
+    bool windowed = round > 0 && (ctx->force_path >= 2 || n_trials >= from);
+    if (windowed) {
+        int rc = ensure(ctx, ctx->rlist, sizeof(int64_t) * n_trials);
+        if (rc == GRC_OK && comp) rc = ensure_bits(ctx);
+        if (rc != GRC_OK && ctx->force_path != 0) return rc;
+        if (rc != GRC_OK) {  // no room for them: the per-trial kernel needs neither
+            windowed = false;
+        }
+    }
+    if (windowed) {
         // projection-window scans (L2-resident map windows) for large trial counts: the warp scan,
         // or the CTA sweep when asked for by grc_set_path(2)
-        TRY(ensure(ctx, ctx->rlist, sizeof(int64_t) * n_trials));
-        if (comp) TRY(ensure_bits(ctx));
         grc::ScoreBufs b = bufs(ctx);
         if (gkey) {  // the windowed kernels fold the first maximum per group in
             b.group_key = gkey;

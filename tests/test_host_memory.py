@@ -29,3 +29,28 @@ def test_a_refused_allocation_is_forgotten(fake):
         assert call() == _lib.GRC_ECUDA
         fake.limit(1 << 40)
         assert call() == _lib.GRC_OK
+
+
+@pytest.mark.parametrize("n,path", [(300, 0), (300, 3), (40000, 0)])
+@pytest.mark.parametrize("median", [False, True])
+def test_no_room_for_the_packed_mask(fake, n, path, median):
+    """Completeness-only calls pack the map, full-output calls list trials for a refine pass; without room for
+    that the per-trial kernel takes them, unless another was asked for."""
+    fake.reset()
+    with fake.context() as ctx:
+        call = scorer(fake, ctx, n)
+        ctx.set_median(median)
+        ctx.set_path(1)
+        assert call() == _lib.GRC_OK           # its own buffers
+        ctx.set_path(path)
+        fake.limit(fake.used() + 256)
+        windowed = not median or path == 3 or n > 1776
+        if path == 3:
+            assert call() == _lib.GRC_ECUDA
+        else:
+            assert call() == _lib.GRC_OK
+            assert ctx.last_stats()["path"] == 1
+        fake.limit(1 << 40)
+        assert call() == _lib.GRC_OK
+        assert ctx.last_stats()["path"] == (3 if windowed else 1)
+        assert fake.stray() == 0
