@@ -216,13 +216,13 @@ __device__ __forceinline__ double spot_cost(const FitFixed &fx, const Beam &e, c
 
 // ---- kernels -------------------------------------------------------------------------
 
-// U*B (9 doubles) of every grain below kFitGrainTable that the spots name, into ub[9 * grain]: a spot
+// U*B (9 doubles) of every grain from 0 to kFitGrainTable that the spots name, into ub[9 * grain]: a spot
 // whose predecessor belongs to another grain writes its grain's (the same values each time).  The
 // entries that take it are not told how many grains there are; a spot of a later grain forms its own.
 __global__ void grain_ub_k(FitFixed fx, const double *grains, SpotList sp, double *ub) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < sp.n; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t gi = sp.grain[i];
-        if ((i > 0 && sp.grain[i - 1] == gi) || gi >= kFitGrainTable) continue;
+        if ((i > 0 && sp.grain[i - 1] == gi) || !in_grain_table(gi)) continue;
         double M[9];
         make_ub(fx, grains + 6 * gi, M);
         for (int k = 0; k < 9; ++k) ub[9 * gi + k] = M[k];
@@ -231,7 +231,7 @@ __global__ void grain_ub_k(FitFixed fx, const double *grains, SpotList sp, doubl
 
 __device__ __forceinline__ void load_ub(const FitFixed &fx, const double *grains, const double *ub, int64_t gi,
                                         double *M) {
-    if (gi < kFitGrainTable) {
+    if (in_grain_table(gi)) {
 #pragma unroll
         for (int k = 0; k < 9; ++k) M[k] = ub[9 * gi + k];
     } else {

@@ -27,6 +27,7 @@ struct SpotList {
 // U*B of the spots' grains: kFitGrainTable x 9 doubles, what the residual, cost and geometry kernels
 // read as `ub`.
 constexpr int64_t kFitGrainTable = 24576;  // 1.8 MB
+__host__ __device__ inline bool in_grain_table(int64_t grain) { return grain >= 0 && grain < kFitGrainTable; }
 cudaError_t fit_grain_ub(const FitFixed &fx, const double *grains, const SpotList &sp, double *ub, cudaStream_t s);
 cudaError_t fit_residual_jacobian(const FitFixed &fx, int mode, const double *grains, const double *ub,
                                   const double *geo10, const SpotList &sp, double *res, double *jac, cudaStream_t s);
