@@ -245,9 +245,8 @@ int set_geometry(grc_ctx *ctx, const float *S, const float *B, const float *hkl,
 }
 
 int upload_device_map(grc_ctx *ctx, const float *d_map, int64_t dz, int64_t dy, int64_t nrot) {
-    const int64_t n = dz * dy * nrot;
     int bad = 0;
-    cudaError_t e = grc::encode_map(d_map, n, ctx->stream, &ctx->mc, ctx->map_ws, &bad);
+    cudaError_t e = grc::encode_map(d_map, dz, dy, nrot, ctx->stream, &ctx->mc, ctx->map_ws, &bad);
     if (e != cudaSuccess) {
         if (!ctx->mc.codes) ctx->has_masks = ctx->bits_ok = false;  // failed while it wrote the map's buffers
         return fail(ctx, GRC_ECUDA, "distance-map coding: %s", cudaGetErrorString(e));
@@ -354,6 +353,23 @@ int stage_geo(grc_ctx *ctx) {
     return GRC_OK;
 }
 
+// Trials from which a call goes to the windowed kernels; `round`: sweep_round_trials.  From a trial per
+// SM on they are faster for every kind of list: a trial per voxel on Al 1537 x 1001 x 121, 500 voxels
+// 0.098 (per-trial kernel) against 0.080 ms, 9,171 0.40 against 0.31; 500 voxels with 1-64 candidates 1.86
+// against 0.32; 256 orientations of one voxel, Al 2048^2 x 361, completeness, 0.127 against 0.088.
+// But a median beyond the 255 distances of the 8-bit codes costs a refine pass, dearer than the trial
+// on the per-trial kernel, which counts 1,024 distances.  Wrong orientations have such medians
+// where spots are far apart: lists wait for half a round there (Fe 1024^2 x 181 with the spots of one
+// grain, a wrong orientation over 300 voxels 0.073 per-trial against 0.161 ms, 4,800 0.334 against 1.13).
+// A middle share of up to 0.4 never had more than one trial in a hundred refined, shares from 0.43 on
+// between none and all.  Scans with medians of 64 orientations and more per voxel, most of them
+// wrong, wait for 1/16 of a round on any map (Fe 1024^2 x 181, 1,024 of one voxel: 0.168 against 0.127 ms
+// without refine passes, 0.153 against 0.381 with; 4,096 without: 0.579 against 0.230).
+int64_t windowed_from(const grc_ctx *ctx, int64_t round, bool list, bool comp) {
+    if (comp || (list && ctx->mc.far_share <= 0.4f)) return ctx->num_sms;
+    return list ? (round + 1) / 2 : (round + 15) / 16;
+}
+
 // Scores n_trials trials into ctx->res.  comp: completeness only (no median; the packed hit mask).
 // gkey (optional): first-maximum keys of every group of gsize consecutive trials, zeroed here.
 int run_score(grc_ctx *ctx, const grc::Work &w, int64_t n_trials, bool comp = false,
@@ -365,15 +381,8 @@ int run_score(grc_ctx *ctx, const grc::Work &w, int64_t n_trials, bool comp = fa
     cudaEvent_t e0 = ctx->timing ? ctx->ev0 : nullptr, e1 = ctx->timing ? ctx->ev1 : nullptr;
     const int64_t round = ctx->force_path == 1 ? 0 : grc::sweep_round_trials(ctx->geo, ctx->num_sms);
     cudaError_t e;
-    // From a trial per SM on the windowed kernels are faster for every kind of list: a trial per voxel
-    // on Al 1537 x 1001 x 121, 500 voxels 0.098 (per-trial kernel) against 0.080 ms, 9,171 0.40 against
-    // 0.31; 500 voxels with 1-64 candidates 1.86 against 0.32; 256 orientations of one voxel, Al 2048^2
-    // x 361, completeness, 0.127 against 0.088.  Scans of one voxel with medians wait for 1/16 of a
-    // round (4,096 on Fe 1024^2 x 181: 0.579 against 0.230): most of their orientations are wrong, and
-    // on a sparse map, with medians beyond 255 distinct distances, a trial's refine pass costs more
-    // than the scan gains (1,024: 0.168 against 0.127 ms without refine passes, 0.153 against 0.381 with).
     const bool shared_voxels = !w.items && !w.trial_voxel && !w.diag && w.n_or >= 64;
-    const int64_t from = shared_voxels && !comp ? (round + 15) / 16 : ctx->num_sms;
+    const int64_t from = windowed_from(ctx, round, !shared_voxels, comp);
     bool fused_key = false;
     bool windowed = round > 0 && (ctx->force_path >= 2 || n_trials >= from);
     if (windowed) {
@@ -1849,9 +1858,9 @@ int batch_enqueue(grc_batch *bt, float *d_out8, float *d_trial_out, int path, in
     w.n_items = m_lim;
     cudaError_t e = cudaSuccess;
     if (T > 0) {
-        // path 1: per-trial kernel; 2: CTA sweep; 3 (and 0 from a trial per SM on): warp scan
+        // path 1: per-trial kernel; 2: CTA sweep; 3 (and 0 from the size for lists on): warp scan
         const int64_t sr = grc::sweep_round_trials(ctx->geo, ctx->num_sms);
-        const int use = sr == 0 ? 1 : (path != 0 ? path : (T >= ctx->num_sms ? 3 : 1));
+        const int use = sr == 0 ? 1 : (path != 0 ? path : (T >= windowed_from(ctx, sr, true, false) ? 3 : 1));
         if (use == 2)
             e = grc::launch_sweep(ctx->geo, b, w, T, ctx->num_sms, ctx->stream, e0, e1, launches, slots);
         else if (use == 3)

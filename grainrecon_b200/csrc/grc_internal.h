@@ -201,14 +201,16 @@ struct MapCodes {
     float *vals = nullptr;
     int64_t n_distinct = 0;
     int code_bits = 0;
+    float far_share = 0;  // of the middle pixels, those with a code that the 8-bit codes hold as 255
     size_t cap_codes = 0, cap_codes8 = 0, cap_vals = 0;  // bytes allocated
     void release();
 };
-// Encodes d_map (n floats) into *resident, whose buffers are reused where they fit.  A map with NaN
+// Encodes d_map (nrot x ny x nz floats) into *resident, whose buffers are reused where they fit.  A map with NaN
 // values (*bad_nan), or a call that fails before the map is known to be good and every buffer
 // allocated, leaves *resident as it is; one that fails after that, with reused buffers partly
 // written, leaves it empty.  ws: two scratches.
-cudaError_t encode_map(const float *d_map, int64_t n, cudaStream_t s, MapCodes *resident, Scratch *ws, int *bad_nan);
+cudaError_t encode_map(const float *d_map, int64_t nz, int64_t ny, int64_t nrot, cudaStream_t s, MapCodes *resident,
+                       Scratch *ws, int *bad_nan);
 
 // Synthetic-data kernels.
 cudaError_t launch_simulate_work(const Geo &g, const ScoreBufs &b, const Work &w, int num_sms, uint8_t *mask,

@@ -494,12 +494,14 @@ int grc_last_stats(grc_ctx *ctx, grc_stats *out);
 /* 1 = record CUDA events around the scoring kernel of each call (for benchmarks). */
 int grc_set_timing(grc_ctx *ctx, int enable);
 /*
- * Scoring kernel selection: 0 = by size (default: the projection-window warp scan, which keeps
+ * Scoring kernel selection: 0 = by size (default): the projection-window warp scan, which keeps
  * the map windows L2-resident and runs one trial per warp at a time, once a call holds a trial per
- * SM -- scans of one voxel with medians 1/16 of a round of trials, 1,776 on 148 SMs; the CTA sweep
- * for full-output calls of more than two rounds on geometries of fewer than 5,000 (projection,
- * reflection) pairs; the per-trial kernel below those
- * sizes), 1 = always the per-trial kernel,
+ * SM; full-output lists on maps with far-apart spots (where wrong orientations have medians beyond
+ * 255 distinct distances) from half a round of trials on, 14,208 on 148 SMs; full-output scans of 64
+ * orientations and more per voxel from 1/16 of a round on, 1,776.  The CTA sweep for full-output calls of
+ * more than two rounds on geometries of fewer than 5,000 (projection, reflection) pairs.  The
+ * per-trial kernel below those sizes, and where the others find no memory for a packed map or a list
+ * of trials.  1 = always the per-trial kernel,
  * 2 = always the CTA sweep (the same windows with the trials of a CTA mixed in its batches),
  * 3 = always the warp scan.  Results are identical; only speed differs.  Batches (grc_batch_*)
  * read the same codes for their tile choice.
