@@ -143,7 +143,9 @@ void apply_options(grc_ctx *ctx) {
     g.Rzf = make_float2((float)(g.R[7] / g.pxy), (float)(g.R[8] / g.pxz));
     g.rpxy = 1.0 / g.pxy;
     g.rpxz = 1.0 / g.pxz;
-    g.Raf = make_float2((float)(g.R[1] / (g.R[0] * g.pxy)), (float)(g.R[2] / (g.R[0] * g.pxz)));
+    // a detector parallel to the beam: K_x reaches u and v through r0 K_x only, which stays a number
+    g.r0 = std::fabs(g.R[0]) >= 1e-20 ? g.R[0] : 1e-20;
+    g.Raf = make_float2((float)(g.R[1] / (g.r0 * g.pxy)), (float)(g.R[2] / (g.r0 * g.pxz)));
     g.beam_stop = g.bsy0 <= g.bsy1 && g.bsy1 >= 1.0 && g.bsy0 <= g.detysize && g.bsz0 <= g.bsz1 && g.bsz1 >= 1.0 &&
                   g.bsz0 <= g.detzsize;
     g.dety0f = (float)g.dety0;

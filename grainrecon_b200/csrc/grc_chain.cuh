@@ -25,7 +25,7 @@ struct OmegaRow {
 // the reflection are folded in (RotDet(1,:) * ax and the pixel scale), plus
 // k_w = Omega^T k_in for the prefilter.
 struct __align__(16) RowF {
-    float cN, ky, kz, L2;   // cN = R(1,1) ax
+    float cN, ky, kz, L2;   // cN = r0 ax, r0 = R(1,1) (Geo)
     float cY, ay, az, num;  // cY = R(1,2) ax / pxy
     float u0, v0, c, s;     // u0 = dety0 - r2d / pxy, v0 = detz0 - r3d / pxz
     float wx, wy, wz, cZ;   // k_w; cZ = R(1,3) ax / pxz
@@ -79,7 +79,7 @@ __device__ __forceinline__ bool in_reach(const Geo &g, const double *__restrict_
 // out of reach gets no u: its landings are all decided in FP64.
 __device__ __forceinline__ RowF row_f32(const Geo &g, const OmegaRow &r, bool reach) {
     RowF f;
-    f.cN = (float)(g.R[0] * r.ax);
+    f.cN = (float)(g.r0 * r.ax);
     f.ky = (float)r.ky; f.kz = (float)r.kz; f.L2 = (float)r.L2;
     f.cY = (float)(g.R[1] * r.ax * g.rpxy);
     f.ay = (float)r.ay; f.az = (float)r.az; f.num = (float)r.num;

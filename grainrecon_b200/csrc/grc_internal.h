@@ -28,8 +28,9 @@ struct Geo {
     // FP32 copies for the fast landing chain
     float Rf[9];
     // ray K -> pixel (u, v): K_y times Ryf = {R[4]/pxy, R[5]/pxz}, K_z times Rzf = {R[7]/pxy, R[8]/pxz}
-    // and R[0] K_x times Raf = {R[1]/(R[0] pxy), R[2]/(R[0] pxz)}
+    // and r0 K_x times Raf = {R[1]/(r0 pxy), R[2]/(r0 pxz)}, r0 = R[0] or, where that is 0, 1e-20
     float2 Ryf, Rzf, Raf;
+    double r0;
     float dety0f, detz0f, rpxyf, rpxzf;
     float half_u, half_v;    // FP32 landings: certain up to here from a pixel's centre (grc_band.h)
     float sin_sure, reach2f; // and up to this sin(theta) and squared distance of the voxel from the rotation axis' origin
