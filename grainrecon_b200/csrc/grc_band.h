@@ -39,10 +39,10 @@ struct Fp32Limits {
 inline Fp32Limits fp32_limits(const Geo &g) {
     const Fp32Limits none{-1.0f, -1.0f, 0.0f, 0.0};
     const double pi = 3.14159265358979323846;
-    for (int i = 0; i < 3; ++i)  // RotDet has to be a rotation for what follows
+    for (int i = 0; i < 3; ++i)  // RotDet has to be a rotation, to two figures, for what follows
         for (int j = 0; j < 3; ++j) {
             const double d = g.R[i] * g.R[j] + g.R[3 + i] * g.R[3 + j] + g.R[6 + i] * g.R[6 + j];
-            if (!(std::fabs(d - (i == j)) <= 1e-3)) return none;
+            if (!(std::fabs(d - (i == j)) <= 1e-2)) return none;
         }
     const double lss = std::fabs(g.lss), lsd = std::fabs(g.lsd);
     const double D0[3] = {g.lsd, g.dety00 - g.rao, g.detz00};

@@ -153,6 +153,15 @@ def test_benchmark_shape_cut_into_pixels(limits, n):
     assert check(g, limits(g), 400000, rng) > 100000
 
 
+@pytest.mark.parametrize("digits", [2, 3, 5])
+def test_rotation_given_to_a_few_digits(limits, digits):
+    rng = np.random.default_rng(digits)
+    g = facing(2048, tilt=3.0)
+    g["R"] = np.round(g["R"], digits)
+    lim = limits(g)
+    assert lim[0] > 0.48 and check(g, lim, 400000, rng) > 100000
+
+
 @pytest.mark.parametrize("seed", range(8))
 def test_random_geometries(limits, seed):
     rng = np.random.default_rng(seed)
