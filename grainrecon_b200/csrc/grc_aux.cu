@@ -191,8 +191,8 @@ __global__ void apply_compete_k(const float *out8, const float *rows5, int64_t m
 // ---- distance-map rank coding --------------------------------------------------
 // Each float maps to an order-preserving 32-bit key; a presence bitmap over the keys plus a prefix
 // popcount gives every value its rank among the distinct values.  A map uses few of the 65,536 upper
-// halves of the keys (distances up to 1,448 pixels: 1,347), so the bitmap holds 65,536 bits for each
-// half in use only: a first pass finds those and numbers them (slots).  The bitmap of all keys took
+// halves of the keys (all distances on 1024 x 1024 pixels: 898), so the bitmap holds 65,536 bits for
+// each half in use only: a first pass finds those and numbers them (slots).  The bitmap of all keys took
 // 1.5 GB with its counts, allocated, cleared and read at every upload; 190 M pixels coded 2.9 -> 1.5 ms
 // (three reads of the map, 0.12 ms each at the copy rate; the rest is the codes' gather of 8 bytes per
 // pixel from L2, 0.72 ms), and the buffers of the map before are used again where they fit.

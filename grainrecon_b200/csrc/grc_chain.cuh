@@ -142,13 +142,12 @@ __device__ void build_gw(const Geo &g, const double *__restrict__ hkl, const dou
 // forward_comp.m:28-59: sin(theta) = -cos(beta), cos(theta) = sin(beta), sin(phiy)
 // expanded, and the ray/plane intersection without normalising K_out.
 __device__ __forceinline__ int64_t landing_fp64(const Geo &g, const OmegaRow &r, double gxw, double gyw,
-                                                double gzw, int iw, double *lam_out = nullptr) {
+                                                double gzw, int iw) {
     // one reciprocal (square root) per length: an FP64 division or square root is some 25 instructions
     const double rG = rsqrt(gxw * gxw + gyw * gyw + gzw * gzw);
     const double Gtx = r.c * gxw - r.s * gyw, Gty = r.s * gxw + r.c * gyw, Gtz = gzw;
     const double x = (r.kx * Gtx + r.ky * Gty + r.kz * Gtz) * rG;  // cos(beta)
     const double lam = 2.0 * (2.0 * CUDART_PI * rG) * (-x);        // 2 d sin(theta)
-    if (lam_out) *lam_out = lam;
     if (!(x < 0.0 && x > g.cbmax && lam > g.lmin && lam < g.lmax)) return -1;
     const double st = -x, ct = sqrt(1.0 - x * x);
     const double s2 = 2.0 * st * ct, c2 = 1.0 - 2.0 * st * st;

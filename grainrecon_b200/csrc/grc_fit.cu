@@ -374,7 +374,7 @@ __device__ __noinline__ bool lm_solve(const double *upper, const double *b, doub
 // at 12 warps per SM: 650 FP64 instructions per spot, cost included, on accumulators in shared
 // memory (in registers: 2 CTAs per SM).  Against dual numbers with 6 tangents in a kernel of their
 // own, two cost kernels and the 6 sines and cosines of the tilts per spot: 5,000 grains of 3,100 spots,
-// two iterations, 7.86 -> 2.1 ms; the spot read one iteration ahead is 2.47 -> 1.89 ms of it.
+// two iterations, 7.87 -> 1.95 ms (2.5 without reading the spot an iteration ahead).
 constexpr int kNE6 = 21 + 6 + 2;
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS, THREADS == 128 ? 3 : 1) grain_lm_k(FitFixed fx, double *grains, const double *geo10, SpotList sp,

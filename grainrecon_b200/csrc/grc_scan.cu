@@ -14,7 +14,7 @@
 //     Lanes hold consecutive projections of a few reflections: their omega rows are consecutive
 //     16-byte words in shared memory, their Gw words broadcasts;
 //   * a selected pixel's map word is read when its batch is evaluated and counted some batches
-//     later: two, in registers, for the bit mask; three, through cp.async, for the 8-bit codes, of
+//     later: two, in registers, for the bit mask; four, through cp.async, for the 8-bit codes, of
 //     which a third miss L2;
 //   * ambiguous items keep their trial in the warp's FP64 queue, drained outside the batch loop: a
 //     call inside it cost 12 spill reloads per batch.
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(kThreads, GRC_SCAN_BLOCKS)
         const uint32_t *wwords = (const uint32_t *)(wcodes - wmis);
         const uint32_t *wbits = MODE == kScanComp ? b.bits + (int64_t)w0 * pw : nullptr;
         // Full mode: the map word of a selected pixel is copied to shared memory when its batch is
-        // evaluated and its code counted kStages - 1 batches later, whichever trials those belong
+        // evaluated and its code counted kStages batches later, whichever trials those belong
         // to, so the gather's latency (a third of the codes miss L2) overlaps their landings.  A byte
         // per batch in flight: 0x80 | bit of the code in its word, or 0; and the batch's trial.
         uint32_t pend = 0, pend_slot = 0;
@@ -598,7 +598,11 @@ cudaError_t launch_scan_t(const Geo &g, const ScoreBufs &b, const Work &w, int64
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     if (win && per_sm > ctas && ctas >= 1) per_sm = ctas;
     const int64_t grid = (int64_t)per_sm * num_sms;
-    // a trial per warp instead of one to two, over many rounds (the lists above: 11.6 -> 11.3 ms)
+    // A trial per warp instead of one to two, over many rounds: the lists above 11.75 -> 11.38 ms; 30,000
+    // voxels with 1-64 candidates on Fe 1024^2 x 181 9.16 -> 7.88, on 2048^2 x 91 5.03 -> 4.21; 100,000
+    // trials of scattered voxels on seven geometries 0-16 % faster.  On Al a voxel per trial is 1-4 %
+    // slower: 30,000 voxels grown 1.69 -> 1.71 ms (2048^2 x 361), 1.68 -> 1.75 (600 x 1900 x 361), 0.655
+    // -> 0.673 (1537 x 1001 x 121; candidates there 4.25 -> 4.31).
     if (MODE == kScanFull && !caller_tile && tile > kWarps && tile < 2 * kWarps && n_trials > 3 * grid * kWarps)
         tile = kWarps;
     // rounds of equal size, so that the last is not a sliver
