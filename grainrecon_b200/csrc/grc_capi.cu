@@ -1990,6 +1990,7 @@ extern "C" int grc_batch_run(grc_batch *bt, float *d_out8, float *d_trial_out) {
     grc_ctx *ctx = bt->ctx;
     Lock l(ctx);
     ctx->stats = grc_stats{};
+    TRY(stage_geo(ctx));  // the options may have changed since the batch was made
     int launches = 0;
     cudaEvent_t e0 = ctx->timing ? ctx->ev0 : nullptr, e1 = ctx->timing ? ctx->ev1 : nullptr;
     TRY(batch_enqueue(bt, d_out8, d_trial_out, bt->path, bt->slots, bt->m, e0, e1, &launches));
@@ -2012,6 +2013,8 @@ extern "C" int grc_batch_capture(grc_batch *bt, float *d_out8) {
         cudaGraphDestroy(bt->graph);
         bt->graph = nullptr;
     }
+    TRY(stage_geo(ctx));
+    CU(cudaStreamSynchronize(ctx->stream));
     CU(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     int launches = 0;
     const int rc = batch_enqueue(bt, d_out8, nullptr, bt->path, bt->slots, bt->m, nullptr, nullptr, &launches);
@@ -2045,6 +2048,7 @@ extern "C" int grc_batch_autotune(grc_batch *bt, float *d_out8, int64_t max_voxe
     if (!bt || !d_out8) return GRC_EINVAL;
     grc_ctx *ctx = bt->ctx;
     Lock l(ctx);
+    TRY(stage_geo(ctx));
     int64_t m_lim = bt->m;
     if (max_voxels > 0 && max_voxels < m_lim) m_lim = max_voxels;
     struct Cand {
