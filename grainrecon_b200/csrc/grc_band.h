@@ -34,8 +34,9 @@ struct Fp32Limits {
 // the axis, source distances of 0.25 to 8 times the detector's.  For detectors that face the source
 // (audited_shape) the error stays below 0.8 of 2.8 (T + W) 2^-24: 0.0039 px on FCC Al 2048^2 and 0.0034 on BCC
 // Fe 1024^2 as benchmarked, where the audit build found no disagreement at half of 0.004 px in 5.8e9
-// decisions.  So 0.004 px is the narrowest band, and the one of those two; 8,192^2 pixels of the
-// same detector take 0.016 px, 32,768^2 0.06, and from some 130,000 a side everything is decided in FP64.
+// decisions.  So 0.004 px is the narrowest band, and the one of those two; the Al detector cut into 8,192^2
+// pixels takes 0.016 px, 32,768^2 0.063, and from 230,000 a side everything is decided in FP64 (Fe, with its
+// larger Bragg angles: 0.007 px at 2,048^2, 0.028 at 8,192^2, all FP64 from 135,000).
 inline Fp32Limits fp32_limits(const Geo &g) {
     const Fp32Limits none{-1.0f, -1.0f, 0.0f, 0.0};
     const double pi = 3.14159265358979323846;
